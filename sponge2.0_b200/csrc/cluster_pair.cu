@@ -19,6 +19,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -34,7 +35,8 @@ constexpr int kWindow = 32;                        // list parts are padded to w
 constexpr unsigned kWordSlotMask = (1u << 22) - 1u; // partner slot field of a list word
 constexpr int kWordMaskShift = 22;                  // the 8-bit atom mask
 constexpr unsigned kWordImage = 1u << 30;           // the pair needs its own periodic image
-constexpr int kPairWarps = 4;                       // warps per block of the force kernel
+constexpr int kListImage = 1 << 30;                 // in a list's length: some word has its image flag set
+constexpr int kPairResident[3] = {28, 20, 12};      // resident warps per SM of the force kernel's modes (registers)
 
 // Per-step slot pack: each slot's offset from the build-time cluster centre
 // moved by the displacement since the build (minimum image in the system's
@@ -176,6 +178,7 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
         unsigned* __restrict__ wc = words + (size_t)c * list_cap;
         const int usable = list_cap - kWindow;  // room left for the padding
         int kh = 0;
+        unsigned any_image = 0;
         for (int t0 = 0; t0 < T; t0 += 32)
         {
             const int t = t0 + lane;
@@ -278,6 +281,7 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
                 if (kh_next <= usable)
                 {
                     if (hit) wc[kh + __popc(mh & below)] = wb | (hit << kWordMaskShift);
+                    any_image |= __any_sync(0xffffffffu, img && hit != 0u);
                 }
                 else if (lane == 0)
                     atomicOr(&counters[kCntOverflow], kOvfWords);
@@ -293,7 +297,7 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
         for (int k2 = kh + lane; k2 < hp; k2 += 32) wc[k2] = null_word;
         if (lane == 0)
         {
-            lcount[s0] = hp;
+            lcount[s0] = hp | (any_image && hp ? kListImage : 0);
             atomicAdd(&kept_total, (unsigned long long)kh);
         }
         __syncwarp();
@@ -320,27 +324,39 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
     }
 }
 
-// Cluster-pair force kernel.  A warp takes clusters from a counter and walks
-// the cluster's list, one word per lane per iteration; the partner's offset
+// Cluster-pair force kernel, one warp a block and one item a warp: a
+// cluster's list, or a part of it.  The warp walks the item's words, one per
+// lane per iteration; the partner's offset
 // {delta + displacement, q} and aux record {22-bit centre, LJ type, global
 // index} load once for all of the cluster's atoms the lane holds, and
 //   dr = (c_J - c_I) * cell / 2^22 + p_j - p_i
 // is formed with the exact integer centre difference.  The cluster's atoms
 // are staged in shared memory as packed pairs, so every instruction of the
-// pair function serves two pairs (FP32x2) and the registers stay few enough
-// for 6 resident blocks per SM (5 with energy/virial totals, 3 with per-atom
-// outputs).  The LJ coefficients of a pair of cluster atoms
-// against the partner's type come as one float4 {-A_a, -A_b, B_a, B_b} of
-// the T^3 table.  Partner records are copied into shared memory by
-// asynchronous copies (cp.async) one iteration ahead of their use, list words
-// two, so their latency overlaps the pair arithmetic.
+// pair function serves two pairs (FP32x2).  The LJ coefficients of a pair of
+// cluster atoms against the partner's type come as one float4
+// {-A_a, -A_b, B_a, B_b} of the T^3 table.  Words are loaded two iterations
+// ahead of their use and partner records one, in registers.
+//
+// What bounds it, and why this shape: a packed FP32x2 instruction holds the
+// FMA pipe for two cycles, and the kernel's time follows the instructions per
+// word, of which only half are the pair arithmetic.  One-warp blocks leave
+// the distribution of the items to the hardware: no counter (an atomic on one
+// address per item), no barrier of unequal warps, no state kept live over the
+// clusters (which spilled), and little shared memory, so that the L1 keeps
+// partner records.  The same kernel as persistent blocks of four warps taking
+// clusters from a counter took 89 us instead of 78 on the 96,000-atom box and
+// 1,317 instead of 1,254 on the 1.0 M-atom box (with the partner records in
+// shared memory rings 91 and 1,364).  Partner sums go out by RED (red_add):
+// the ATOMG that atomicAdd becomes here waits for an answer, and with it and
+// a test per component instead of one per word the two boxes took 103 and
+// 1,548, the per-atom mode 217 instead of 151.
 //
 // Each pair is evaluated once; a lane holds all 8 atoms, the partner's force
 // (summed over the 8 in a fixed order) goes to its int64 fixed-point
 // accumulator by one atomic add per component and word, and the cluster's
-// forces are summed over the lanes as int64 and added the same way.  Integer
-// addition does not depend on order, so the forces are bitwise reproducible;
-// the finishing pass converts them.
+// forces are summed over the lanes in FP64 in a fixed order and added the same
+// way.  Integer addition does not depend on order, so the forces are bitwise
+// reproducible; the finishing pass converts them.
 //
 // MODE 0: forces.  MODE 1: + energy and virial totals.  MODE 2: + per-atom
 // energy and virial: a pair's terms belong to its owner, the atom with the
@@ -350,145 +366,103 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
 // partner-owned sums go to the partner's int64 staging, 8 atomic adds; the
 // finishing pass turns the staging into the per-atom arrays and totals.
 template <int MODE, int FIT, bool TRI>
-__global__ void __launch_bounds__(kPairWarps * 32, MODE == 2 ? 3 : (MODE == 1 ? 5 : 7))
+__global__ void __launch_bounds__(32, kPairResident[MODE])
     k_pair8(ForceParams p0, const ForceParams* __restrict__ fps, const SysDesc* __restrict__ sys, int n_clusters,
-            int list_cap, const int* __restrict__ cl_sys, const int* __restrict__ lcount,
+            int shift, int list_cap, const int* __restrict__ cl_sys, const int* __restrict__ lcount,
             const unsigned* __restrict__ words, const int4* __restrict__ cl_q, const float4* __restrict__ pos,
             const int4* __restrict__ aux, const float4* __restrict__ t4, long long* __restrict__ facc,
-            long long* __restrict__ oacc, long long* __restrict__ totals, const int* __restrict__ only,
-            int* __restrict__ counters, int max_types)
+            long long* __restrict__ oacc, long long* __restrict__ totals, const int* __restrict__ only)
 {
     grid_dep_wait();
     constexpr bool EN = MODE >= 1;
     constexpr bool PA = MODE >= 2;
     constexpr int NP = 4;        // the cluster's 8 atoms as packed pairs
-    __shared__ long long red[kPairWarps][8];  // per-warp fixed-point totals
-    __shared__ int is_last;
-    extern __shared__ float4 rows_all[];      // per warp: 4 x max_types coefficient rows
-    __shared__ unsigned wring_all[kPairWarps][3][32];       // per warp: list words in flight
-    // per warp: the cluster's atom pairs {-x, -y | -z, q} and global indices
-    __shared__ float4 iat_all[kPairWarps][4][2];
-    __shared__ int2 igid_all[kPairWarps][4];
-    __shared__ __align__(16) float4 jpos_all[kPairWarps][2][32];  // partner offsets and charges in flight
-    __shared__ __align__(16) int4 jaux_all[kPairWarps][2][32];    // partner aux records in flight
-    const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
-    float4* __restrict__ rows = rows_all + w * 4 * max_types;
-    unsigned(&wring)[3][32] = wring_all[w];
-    float4(&iat)[4][2] = iat_all[w];
-    int2(&igid)[4] = igid_all[w];
-    float4(&jpos)[2][32] = jpos_all[w];
-    int4(&jaux)[2][32] = jaux_all[w];
-    if (EN && lane < 8) red[w][lane] = 0;
-    __syncwarp();
-    int cur_sys = -1;  // the system red[w] accumulates for
-    for (;;)
+    extern __shared__ float4 rows[];  // 4 x types coefficient rows (at least 8 x kSumRow floats)
+    float* sums = reinterpret_cast<float*>(rows);  // after the list, the lanes' sums
+    __shared__ float4 iat[4][2];  // the cluster's atom pairs {-x, -y | -z, -q}
+    __shared__ int2 igid[4];      // and their global indices
+    const int lane = threadIdx.x;
+    // the item: part blockIdx.x mod 2^shift of the windows of its cluster's list
+    const int c = blockIdx.x >> shift, part = blockIdx.x & ((1 << shift) - 1);
+    const int s0 = c * kClusterSize;
+    const int head = lcount[s0];
+    const int windows = (head & ~kListImage) / kWindow;
+    const int it0 = (windows * part) >> shift;
+    const int iters = ((windows * (part + 1)) >> shift) - it0;
+    if (iters <= 0) return;
+    const int sy = cl_sys[c];
+    if (only && !only[sy]) return;
+    const ForceParams P = fps ? fps[sy] : p0;
+    const PairParams2 pp = pack_params(P);
+    const SysDesc& D = sys[sy];
+    const Cell qc = D.qcell;
+    const int slot0 = D.cl_begin * kClusterSize;
+    const int4 ci = cl_q[c];
+    const int nt = P.n_types;
+    // the cluster's atoms, negated, as packed pairs, and the coefficient
+    // rows of its four atom pairs against every partner type,
+    // {-A_a, -A_b, B_a, B_b}, staged in shared memory
     {
-        int c = 0;
-        if (lane == 0) c = atomicAdd(&counters[kCntPairNext], 1);
-        c = __shfl_sync(0xffffffffu, c, 0);
-        if (c >= n_clusters) break;
-        const int s0 = c * kClusterSize;
-        const int total = lcount[s0];  // a multiple of the window
-        if (total == 0) continue;
-        const int sy = cl_sys[c];
-        if (only && !only[sy]) continue;
-        if (EN && sy != cur_sys)
+        const float4 u = pos[s0 + (lane & 7)];
+        const int4 x = aux[s0 + (lane & 7)];
+        if (lane < 8)
         {
-            // totals belong to one system each: flush this warp's share
-            __syncwarp();
-            if (lane == 0 && cur_sys >= 0)
-                for (int q = 0; q < 8; q++)
-                {
-                    const long long v = red[w][q];
-                    if (v) atomicAdd((unsigned long long*)&totals[8 * cur_sys + q], (unsigned long long)v);
-                    red[w][q] = 0;
-                }
-            __syncwarp();
-            cur_sys = sy;
+            float* f = reinterpret_cast<float*>(&iat[lane >> 1][0]) + (lane & 1);
+            f[0] = -u.x;
+            f[2] = -u.y;
+            f[4] = -u.z;
+            f[6] = -u.w;
+            if (PA) reinterpret_cast<int*>(&igid[lane >> 1])[lane & 1] = x.w;
         }
-        const ForceParams P = fps ? fps[sy] : p0;
-        const PairParams2 pp = pack_params(P);
-        const SysDesc& D = sys[sy];
-        const Cell qc = D.qcell;
-        const int slot0 = D.cl_begin * kClusterSize;
-        const int4 ci = cl_q[c];
-        const int nt = P.n_types;
-        // the cluster's atoms, negated, as packed pairs
-        __syncwarp();  // the previous cluster's atoms are no longer read
-        if (lane < 4)
+        const int ti = (x.x >> 22) & 0x7f;
+        const int row = (ti * nt + __shfl_down_sync(0xffffffffu, ti, 1)) * nt;  // of lanes 0, 2, 4, 6
+        const float4* __restrict__ r = t4 + P.t4_begin;
+#pragma unroll
+        for (int q = 0; q < 4; q++)
         {
-            const int a = 2 * lane;
-            const float4 u0 = pos[s0 + a], u1 = pos[s0 + a + 1];
-            iat[lane][0] = make_float4(-u0.x, -u1.x, -u0.y, -u1.y);
-            iat[lane][1] = make_float4(-u0.z, -u1.z, u0.w, u1.w);
-            igid[lane] = make_int2(aux[s0 + a].w, aux[s0 + a + 1].w);
+            const int first = __shfl_sync(0xffffffffu, row, 2 * q);
+            for (int e = lane; e < nt; e += 32) rows[q * nt + e] = __ldg(r + first + e);
         }
-        __syncwarp();
-        // the coefficient rows of the cluster's four atom pairs against every
-        // partner type, {-A_a, -A_b, B_a, B_b}, staged in shared memory
-        {
-            int rq[4];
+    }
+    __syncwarp();
+    float2 fx[NP], fy[NP], fz[NP];
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                rq[q] = P.t4_begin + (((aux[s0 + 2 * q].x >> 22) & 0x7f) * nt + ((aux[s0 + 2 * q + 1].x >> 22) & 0x7f)) * nt;
-            __syncwarp();  // the previous cluster's rows are no longer read
-            for (int e = lane; e < 4 * nt; e += 32)
-            {
-                const int q = e / nt;
-                const int r = q == 0 ? rq[0] : (q == 1 ? rq[1] : (q == 2 ? rq[2] : rq[3]));
-                rows[e] = __ldg(t4 + r + (e - q * nt));
-            }
-            __syncwarp();
-        }
-        float2 fx[NP], fy[NP], fz[NP];
+    for (int p = 0; p < NP; p++) fx[p] = fy[p] = fz[p] = f2(0.0f);
+    float2 acc[(EN && !PA) ? 8 : 1];
 #pragma unroll
-        for (int p = 0; p < NP; p++) fx[p] = fy[p] = fz[p] = f2(0.0f);
-        float2 acc[(EN && !PA) ? 8 : 1];
+    for (int q = 0; q < ((EN && !PA) ? 8 : 1); q++) acc[q] = f2(0.0f);
+    float2 own[PA ? NP : 1][PA ? 8 : 1];
 #pragma unroll
-        for (int q = 0; q < ((EN && !PA) ? 8 : 1); q++) acc[q] = f2(0.0f);
-        float2 own[PA ? NP : 1][PA ? 8 : 1];
+    for (int p = 0; p < (PA ? NP : 1); p++)
 #pragma unroll
-        for (int p = 0; p < (PA ? NP : 1); p++)
-#pragma unroll
-            for (int q = 0; q < (PA ? 8 : 1); q++) own[p][q] = f2(0.0f);
+        for (int q = 0; q < (PA ? 8 : 1); q++) own[p][q] = f2(0.0f);
 
-        const unsigned* __restrict__ wb = words + (size_t)c * list_cap;
-        // a three-deep ring of list words and a two-deep ring of partner
-        // records in shared memory, filled by asynchronous copies: a lane
-        // only ever reads what it copied itself, so no warp barrier is needed
-        auto stage_word = [&](int it) {
-            if (it * 32 < total) cp_async(&wring[it % 3][lane], wb + it * 32 + lane, 4);
-            cp_async_commit();
-        };
-        auto stage_partner = [&](int it, unsigned w) {
-            if (it * 32 < total)
-            {
-                const int j = slot0 + (int)(w & kWordSlotMask);
-                cp_async(&jpos[it & 1][lane], pos + j, 16);
-                cp_async(&jaux[it & 1][lane], aux + j, 16);
-            }
-            cp_async_commit();
-        };
-        const int iters = total / 32;
-        stage_word(0);
-        stage_word(1);
-        cp_async_wait_prior();
-        unsigned wc = wring[0][lane];
-        stage_partner(0, wc);
+    const unsigned* __restrict__ wb = words + (size_t)c * list_cap + kWindow * it0;
+    // the list's words; IMG: some of them need their pairs' own images
+    auto walk = [&](auto image) {
+        constexpr bool IMG = decltype(image)::value;
+        // list words are loaded two iterations ahead of their use and
+        // partner records one ahead, in registers
+        const unsigned* __restrict__ wl = wb + lane;
+        unsigned wc = wl[0];
+        unsigned wn = iters > 1 ? wl[32] : 0u;
+        float4 pjn = pos[slot0 + (int)(wc & kWordSlotMask)];
+        int4 xjn = aux[slot0 + (int)(wc & kWordSlotMask)];
 #pragma unroll 1
         for (int it = 0; it < iters; it++)
         {
-            // in flight, oldest first: word it+1, partner it, then word it+2
-            stage_word(it + 2);
-            cp_async_wait_prior();
-            const unsigned wn = wring[(it + 1) % 3][lane];
-            const float4 pjc = jpos[it & 1][lane];
-            const int4 xjc = jaux[it & 1][lane];
+            const float4 pjc = pjn;
+            const int4 xjc = xjn;
             const int jc = slot0 + (int)(wc & kWordSlotMask);
-            stage_partner(it + 1, wn);
+            unsigned wnn = 0u;
+            if (it + 1 < iters)
+            {
+                const int jn = slot0 + (int)(wn & kWordSlotMask);
+                pjn = pos[jn];
+                xjn = aux[jn];
+                if (it + 2 < iters) wnn = wl[32 * (it + 2)];
+            }
 
-            const unsigned mi = (wc >> kWordMaskShift) & 0xffu;
             const float ux = centre_step(xjc.x, ci.x), uy = centre_step(xjc.y, ci.y), uz = centre_step(xjc.z, ci.z);
             // the partner in the frame of the cluster's centre
             float sx = __fmaf_rn(ux, qc.a11, pjc.x);
@@ -500,12 +474,10 @@ __global__ void __launch_bounds__(kPairWarps * 32, MODE == 2 ? 3 : (MODE == 1 ? 
                 sx = __fmaf_rn(uz, qc.a31, sx);
                 sy2 = __fmaf_rn(uz, qc.a32, sy2);
             }
-            const bool img = (wc & kWordImage) != 0u;
-            const bool any_img = __any_sync(0xffffffffu, img);
             const int tj = (xjc.x >> 22) & 0x7f;
             const int gj = xjc.w;
             const float2 qj = f2(pjc.w);
-            float2 hx = f2(0.0f), hy = f2(0.0f), hz = f2(0.0f);  // the partner's force, negated
+            float2 hx, hy, hz;     // the partner's force, negated
             float2 jo[PA ? 8 : 1];                                  // the partner's owned sums
 #pragma unroll
             for (int q = 0; q < (PA ? 8 : 1); q++) jo[q] = f2(0.0f);
@@ -516,7 +488,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, MODE == 2 ? 3 : (MODE == 1 ? 
                 const float2 pnx = make_float2(A.x, A.y), pny = make_float2(A.z, A.w), pnz = make_float2(B.x, B.y),
                              pq = make_float2(B.z, B.w);
                 float2 dx = __fadd2_rn(f2(sx), pnx), dy = __fadd2_rn(f2(sy2), pny), dz = __fadd2_rn(f2(sz), pnz);
-                if (any_img && img)
+                if (IMG && (wc & kWordImage))
                 {
                     // small box: the pair takes its own minimum image
                     float ddx[2] = {dx.x, dx.y}, ddy[2] = {dy.x, dy.y}, ddz[2] = {dz.x, dz.y};
@@ -535,20 +507,20 @@ __global__ void __launch_bounds__(kPairWarps * 32, MODE == 2 ? 3 : (MODE == 1 ? 
                     dz = make_float2(ddz[0], ddz[1]);
                 }
                 const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-                const bool inA = ((mi >> (2 * p)) & 1u) && r2.x < pp.rc2;
-                const bool inB = ((mi >> (2 * p + 1)) & 1u) && r2.y < pp.rc2;
+                const bool inA = (wc & (1u << (kWordMaskShift + 2 * p))) && r2.x < pp.rc2;
+                const bool inB = (wc & (2u << (kWordMaskShift + 2 * p))) && r2.y < pp.rc2;
                 const float4 ab = rows[p * nt + tj];
                 float2 elj, ec;
                 float2 f = pair_scalar2<EN, FIT>(r2, __fmul2_rn(qj, pq), make_float2(ab.x, ab.y),
                                                  make_float2(ab.z, ab.w), pp, elj, ec);
                 f = make_float2(inA ? f.x : 0.0f, inB ? f.y : 0.0f);
-                const float2 gx = __fmul2_rn(f, dx), gy = __fmul2_rn(f, dy), gz = __fmul2_rn(f, dz);
-                fx[p] = __fadd2_rn(fx[p], gx);
-                fy[p] = __fadd2_rn(fy[p], gy);
-                fz[p] = __fadd2_rn(fz[p], gz);
-                hx = __fadd2_rn(hx, gx);
-                hy = __fadd2_rn(hy, gy);
-                hz = __fadd2_rn(hz, gz);
+                fx[p] = __ffma2_rn(f, dx, fx[p]);
+                fy[p] = __ffma2_rn(f, dy, fy[p]);
+                fz[p] = __ffma2_rn(f, dz, fz[p]);
+                hx = p == 0 ? __fmul2_rn(f, dx) : __ffma2_rn(f, dx, hx);
+                hy = p == 0 ? __fmul2_rn(f, dy) : __ffma2_rn(f, dy, hy);
+                hz = p == 0 ? __fmul2_rn(f, dz) : __ffma2_rn(f, dz, hz);
+                const float2 gx = __fmul2_rn(f, dx), gy = __fmul2_rn(f, dy), gz = __fmul2_rn(f, dz);  // the virial's
                 if (EN && !PA)
                 {
                     acc[0] = __fadd2_rn(acc[0], make_float2(inA ? elj.x : 0.0f, inB ? elj.y : 0.0f));
@@ -593,107 +565,84 @@ __global__ void __launch_bounds__(kPairWarps * 32, MODE == 2 ? 3 : (MODE == 1 ? 
                 }
                 if (any)
                 {
-                    unsigned long long* oa = (unsigned long long*)(oacc + jc);
+                    long long* oa = oacc + jc;
                     const size_t ostride = (size_t)n_clusters * kClusterSize;
 #pragma unroll
                     for (int q = 0; q < 8; q++)
-                    {
-                        const long long v = __float2ll_rn(js[q] * kTwoPow32);
-                        if (v) atomicAdd(oa + q * ostride, (unsigned long long)v);
-                    }
+                        red_add(oa + q * ostride, __float2ll_rn(js[q] * kTwoPow32));
                 }
             }
             {
                 // the partner's force: minus the sum over the cluster's atoms
-                const long long qx = __float2ll_rn(-(hx.x + hx.y) * kTwoPow32);
-                const long long qy = __float2ll_rn(-(hy.x + hy.y) * kTwoPow32);
-                const long long qz = __float2ll_rn(-(hz.x + hz.y) * kTwoPow32);
-                unsigned long long* fa = (unsigned long long*)(facc + 3 * (size_t)jc);
-                if (qx) atomicAdd(fa + 0, (unsigned long long)qx);
-                if (qy) atomicAdd(fa + 1, (unsigned long long)qy);
-                if (qz) atomicAdd(fa + 2, (unsigned long long)qz);
+                // (all zero when the word has no pair inside the cutoff)
+                const float jx = hx.x + hx.y, jy = hy.x + hy.y, jz = hz.x + hz.y;
+                if (jx != 0.0f || jy != 0.0f || jz != 0.0f)
+                {
+                    long long* fa = facc + 3 * (size_t)jc;
+                    red_add(fa + 0, __float2ll_rn(jx * -kTwoPow32));
+                    red_add(fa + 1, __float2ll_rn(jy * -kTwoPow32));
+                    red_add(fa + 2, __float2ll_rn(jz * -kTwoPow32));
+                }
             }
             wc = wn;
+            wn = wnn;
         }
-        cp_async_wait_all();
+    };
+    if (head & kListImage)
+        walk(std::true_type{});
+    else
+        walk(std::false_type{});
 
-        // the cluster's forces: int64 per lane, summed over the lanes by a
-        // reduce-scatter (lanes 4a..4a+3 end with atom a)
-        long long vx[8], vy[8], vz[8];
+    // the cluster's sums over the lanes, eight at a time: lane 4a + d takes
+    // component d of atom a's force; in the totals mode lane 4q + 3 the
+    // energy or virial q
+    double sum = 0.0;
+#pragma unroll
+    for (int d = 0; d < (EN && !PA ? 4 : 3); d++)
+    {
+        float v[8];
 #pragma unroll
         for (int a = 0; a < 8; a++)
         {
-            const int p = a / 2;
-            const float sxv = (a & 1) ? fx[p].y : fx[p].x, syv = (a & 1) ? fy[p].y : fy[p].x,
-                        szv = (a & 1) ? fz[p].y : fz[p].x;
-            vx[a] = __float2ll_rn(sxv * kTwoPow32);
-            vy[a] = __float2ll_rn(syv * kTwoPow32);
-            vz[a] = __float2ll_rn(szv * kTwoPow32);
+            const float2 u = d == 0 ? fx[a / 2] : (d == 1 ? fy[a / 2] : fz[a / 2]);
+            v[a] = d == 3 ? acc[a % ((EN && !PA) ? 8 : 1)].x + acc[a % ((EN && !PA) ? 8 : 1)].y : ((a & 1) ? u.y : u.x);
         }
-        const long long Fx = reduce_scatter8(vx, lane), Fy = reduce_scatter8(vy, lane),
-                        Fz = reduce_scatter8(vz, lane);
-        const int va = lane >> 2;
-        if ((lane & 3) == 0)
-        {
-            unsigned long long* fa = (unsigned long long*)(facc + 3 * (size_t)(s0 + va));
-            if (Fx) atomicAdd(fa + 0, (unsigned long long)Fx);
-            if (Fy) atomicAdd(fa + 1, (unsigned long long)Fy);
-            if (Fz) atomicAdd(fa + 2, (unsigned long long)Fz);
-        }
-        if (EN && !PA)
-        {
-            float ev[8];
+        const double s = lane_totals8(sums, v, lane);
+        if ((lane & 3) == d) sum = s;
+    }
+    if ((lane & 3) < 3)
+        red_add(facc + 3 * (size_t)(s0 + (lane >> 2)) + (lane & 3), __double2ll_rn(sum * kForceScale));
+    else if (EN && !PA)
+    {
+        // each pair once; the virial is -g (x) d, its symmetric
+        // off-diagonal terms (xy + yx etc.) twice the one accumulated
+        const int q = lane >> 2;
+        const double sc = q == 0 ? (double)kLjEnergyScale
+                                 : (q == 1 ? (double)kCoulombEnergyScale
+                                           : ((q == 3 || q == 5 || q == 6) ? -2.0 : -1.0));
+        red_add(totals + 8 * (size_t)sy + q, __double2ll_rn(sum * sc * kEnergyScale));
+    }
+    if (PA)
+    {
+        // the cluster's owned sums: raw fixed point to each atom's
+        // staging (scaled in the finishing pass), lane 4a + k quantity
+        // q0 + k of atom a
 #pragma unroll
-            for (int q = 0; q < 8; q++) ev[q] = acc[q].x + acc[q].y;
-            const float esum = reduce_scatter8(ev, lane);
-            if ((lane & 3) == 0)
-            {
-                // each pair once; the virial is -g (x) d, its symmetric
-                // off-diagonal terms (xy + yx etc.) twice the one accumulated
-                const double sc = va == 0 ? (double)kLjEnergyScale
-                                          : (va == 1 ? 1.0 : ((va == 3 || va == 5 || va == 6) ? -2.0 : -1.0));
-                red[w][va] += __double2ll_rn((double)esum * sc * kEnergyScale);
-            }
-        }
-        if (PA)
+        for (int q0 = 0; q0 < 8; q0 += 4)
         {
-            // the cluster's owned sums: raw fixed point to each atom's
-            // staging (scaled in the finishing pass)
+            double o = 0.0;
 #pragma unroll
-            for (int a = 0; a < 8; a++)
+            for (int k = 0; k < 4; k++)
             {
-                const int p = a / 2;
                 float v[8];
 #pragma unroll
-                for (int q = 0; q < 8; q++) v[q] = (a & 1) ? own[p][q].y : own[p][q].x;
-                // lanes 4q..4q+3 end with value q of atom a
-                const float val = reduce_scatter8(v, lane);
-                const long long r = __float2ll_rn(val * kTwoPow32);
-                if ((lane & 3) == 0 && r)
-                    atomicAdd((unsigned long long*)(oacc + (size_t)va * n_clusters * kClusterSize + (s0 + a)),
-                              (unsigned long long)r);
+                for (int a = 0; a < 8; a++) v[a] = (a & 1) ? own[a / 2][q0 + k].y : own[a / 2][q0 + k].x;
+                const double s = lane_totals8(sums, v, lane);
+                if ((lane & 3) == k) o = s;
             }
+            red_add(oacc + (size_t)(q0 + (lane & 3)) * n_clusters * kClusterSize + s0 + (lane >> 2),
+                    __double2ll_rn(o * kForceScale));
         }
-    }
-    __syncwarp();
-    if (EN && lane == 0 && cur_sys >= 0)
-        for (int q = 0; q < 8; q++)
-        {
-            const long long v = red[w][q];
-            if (v) atomicAdd((unsigned long long*)&totals[8 * cur_sys + q], (unsigned long long)v);
-        }
-    // the last block resets the cluster counter for the next launch
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        __threadfence();
-        is_last = atomicAdd(&counters[kCntPairDone], 1) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (is_last && threadIdx.x == 0)
-    {
-        counters[kCntPairNext] = 0;
-        counters[kCntPairDone] = 0;
     }
 }
 
@@ -862,14 +811,14 @@ __global__ void k_fin8_atoms(int n, int slots, const int* __restrict__ atom_slot
 #pragma unroll
                 for (int u = 0; u < 8; u++) oacc[(size_t)u * slots + sl[k]] = 0;
             }
-        // raw sums: -12 E_lj, E_c, and +g (x) d; the virial is -g (x) d with
+        // raw sums: -12 E_lj, -E_c, and +g (x) d; the virial is -g (x) d with
         // the symmetric off-diagonal terms twice the one summed
         double v[8];
 #pragma unroll
         for (int u = 0; u < 8; u++)
         {
             const double sg = u == 0 ? (double)kLjEnergyScale
-                                     : (u == 1 ? 1.0 : ((u == 3 || u == 5 || u == 6) ? -2.0 : -1.0));
+                                     : (u == 1 ? (double)kCoulombEnergyScale : ((u == 3 || u == 5 || u == 6) ? -2.0 : -1.0));
             v[u] = (double)r[u] * sg;
             tq[u] = __double2ll_rn(v[u]);
         }
@@ -928,35 +877,34 @@ __global__ void k_fin8_atoms(int n, int slots, const int* __restrict__ atom_slot
     }
 }
 
-// A persistent grid: as many blocks as can be resident on every SM.
-template <typename K>
-int resident_blocks(K kernel, int threads, size_t smem)
-{
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess ||
-        per_sm <= 0)
-    {
-        cudaGetLastError();
-        per_sm = 4;
-    }
-    return per_sm * num_sms();
-}
-
 template <int M, int F, bool T>
 int launch_pair(const ForceInputs& in, cudaStream_t s)
 {
     const spgnb_nl* nl = in.nl;
     const int mt = in.max_types > 0 ? in.max_types : in.p0.n_types;
-    const size_t smem = sizeof(float4) * kPairWarps * 4 * mt;
-    int resident = resident_blocks(k_pair8<M, F, T>, kPairWarps * 32, smem);
-    if (in.pair_blocks_per_sm > 0) resident = std::min(resident, in.pair_blocks_per_sm * num_sms());
-    const int grid = std::max(1, std::min(resident, (nl->clusters_cap + kPairWarps - 1) / kPairWarps));
+    size_t smem = sizeof(float4) * std::max(4 * mt, 2 * kSumRow);
+    // the blocks-per-SM setting counts blocks of four warps: it holds the
+    // resident ones down by the shared memory each asks for
+    if (in.pair_blocks_per_sm > 0)
+        smem = std::max(smem, (size_t)(220 * 1024 / (4 * in.pair_blocks_per_sm)) & ~(size_t)127);
+    // Each cluster's list in 2^shift parts, as many as keep the items within
+    // one and a half times the warps the chip holds.  With fewer clusters than
+    // warps the kernel's time is one warp's walk over a list: the 6,480-atom
+    // box takes 39 us with whole lists and 14 with four parts, the 1,944-atom
+    // one 26 and 7.  An item costs about one and a half windows of its own
+    // (the 96,000-atom box takes 80 us with whole lists, 82 with halves, 101
+    // with quarters).  Several systems: whole lists, since a system's sums, and
+    // with them its trajectory's bits, must not depend on the systems around it.
+    int shift = 0;
+    if (!in.d_fps)
+        while (shift < 4 && ((long long)nl->clusters_cap << (shift + 1)) <= 3LL * kPairResident[M] * num_sms() / 2) shift++;
+    const unsigned grid = (unsigned)nl->clusters_cap << shift;
     if (smem > 48 * 1024)
         SPGNB_CUDA(cudaFuncSetAttribute(k_pair8<M, F, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)smem));
-    launch_dependent(k_pair8<M, F, T>, grid, kPairWarps * 32, smem, s,
-        in.p0, in.d_fps, nl->d_sys, nl->clusters_cap, nl->list_cap, nl->d_cl_sys, nl->d_pcount, nl->d_pwords,
-        nl->d_cl_q, in.slot_pos, in.slot_aux, in.t4, nl->d_facc, nl->d_oacc, in.totals, in.only, nl->d_counters, mt);
+    launch_dependent(k_pair8<M, F, T>, grid, 32, smem, s,
+        in.p0, in.d_fps, nl->d_sys, nl->clusters_cap, shift, nl->list_cap, nl->d_cl_sys, nl->d_pcount, nl->d_pwords,
+        nl->d_cl_q, in.slot_pos, in.slot_aux, in.t4, nl->d_facc, nl->d_oacc, in.totals, in.only);
     SPGNB_CHECK_LAUNCH("k_pair8");
     return SPGNB_OK;
 }

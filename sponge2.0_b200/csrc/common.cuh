@@ -136,8 +136,6 @@ enum Counter
     kCntPWordsLast = 16,  // 64-bit: words of the last completed pruning (slots 16,17)
     kCntPruneNext = 18,   // the next cluster a warp of the running prune kernel takes
     kCntSearchNext = 19,  // the next cluster a warp of the running search kernel takes
-    kCntPairNext = 20,    // the next cluster a warp of the running force kernel takes
-    kCntPairDone = 21,    // blocks of the running force kernel that finished
     kCntSize = 24
 };
 

@@ -57,17 +57,18 @@ enum PackedConst
 {
     kPkMinusOne = 0
 };
-// pair_scalar2's LJ energy is -12 times the energy (A/(12 r^12) - B/(6 r^6)):
-// the kernels scale the sums once
+// pair_scalar2's LJ energy is -12 times the energy (A/(12 r^12) - B/(6 r^6))
+// and its Coulomb energy -1 times the energy: the kernels scale the sums once
 constexpr float kLjEnergyScale = -1.0f / 12.0f;
+constexpr float kCoulombEnergyScale = -1.0f;
 
-__device__ __forceinline__ float2 poly5x2(float2 x, const float2* c)
+template <int N>
+__device__ __forceinline__ float2 polyx2(float2 x, const float2 (&c)[N])
 {
-    float2 p = __ffma2_rn(c[5], x, c[4]);
-    p = __ffma2_rn(p, x, c[3]);
-    p = __ffma2_rn(p, x, c[2]);
-    p = __ffma2_rn(p, x, c[1]);
-    return __ffma2_rn(p, x, c[0]);
+    float2 p = c[N - 1];
+#pragma unroll
+    for (int k = N - 2; k >= 0; k--) p = __ffma2_rn(p, x, c[k]);
+    return p;
 }
 
 __device__ __forceinline__ float ex2_approx(float x)
@@ -116,12 +117,15 @@ __device__ __forceinline__ PairParams2 pack_params(const ForceParams& pc)
     return q;
 }
 
-// pair_scalar for two pairs at once; nA = -A.  Without energies the screened
-// Coulomb force uses the K fit; with energies it uses the M fit and
-// exp(-w): beta^3 K(w) = beta (M(w) - 2/sqrt(pi) exp(-w)) / r^2, so
+// pair_scalar for two pairs at once; nA = -A, nqq = -q_i q_j (the kernels keep
+// a cluster's charges negated), so that the Coulomb term joins the LJ term in
+// one fused multiply-add.  Without energies the screened Coulomb force uses
+// the K fit; with energies it uses the M fit and exp(-w):
+// beta^3 K(w) = beta (M(w) - 2/sqrt(pi) exp(-w)) / r^2, so
 //   F_c/qq = (t + beta 2/sqrt(pi) exp(-w)) / r^2,  E_c/qq = t,  t = 1/r - beta M(w).
+// e_lj comes out as -12 E_lj and e_c as -E_c; the kernels scale the sums once.
 template <bool ENERGY, int FIT>
-__device__ __forceinline__ float2 pair_scalar2(float2 r2, float2 qq, float2 nA, float2 B, const PairParams2& pc,
+__device__ __forceinline__ float2 pair_scalar2(float2 r2, float2 nqq, float2 nA, float2 B, const PairParams2& pc,
                                                float2& e_lj, float2& e_c)
 {
     // the hardware reciprocal square root alone: a Newton step on top of it
@@ -132,45 +136,36 @@ __device__ __forceinline__ float2 pair_scalar2(float2 r2, float2 qq, float2 nA, 
     const float2 r6inv = __fmul2_rn(__fmul2_rn(r2inv, r2inv), r2inv);
     // u = (-A/r^6 + B)/r^6 serves the force and, plus B/r^6, the energy
     const float2 u = __fmul2_rn(__ffma2_rn(nA, r6inv, B), r6inv);
-    const float2 flj = __fmul2_rn(u, r2inv);
-    float2 fc;
+    if (ENERGY) e_lj = __ffma2_rn(B, r6inv, u);  // -A/r^12 + 2B/r^6 = -12 E_lj
     if (FIT == 1)
     {
         const float2 x = __fmul2_rn(r2, pc.w_scale);
         if (!ENERGY)
         {
-            const float2 kp = poly5x2(x, kEwaldKP2), kq = poly5x2(x, kEwaldKQ2);
+            const float2 kp = polyx2(x, kEwaldKP2), kq = polyx2(x, kEwaldKQ2);
             const float2 K = __fmul2_rn(kp, make_float2(rcp_approx(kq.x), rcp_approx(kq.y)));
-            fc = __fmul2_rn(qq, __ffma2_rn(pc.nbeta3, K, __fmul2_rn(rinv, r2inv)));
+            return __ffma2_rn(nqq, __ffma2_rn(pc.nbeta3, K, __fmul2_rn(rinv, r2inv)), __fmul2_rn(u, r2inv));
         }
-        else
-        {
-            const float2 mp = poly5x2(x, kEwaldMP2), mq = poly5x2(x, kEwaldMQ2);
-            const float2 M = __fmul2_rn(mp, make_float2(rcp_approx(mq.x), rcp_approx(mq.y)));
-            const float2 wl = __fmul2_rn(r2, pc.nb2_log2e);
-            const float2 E = make_float2(ex2_approx(wl.x), ex2_approx(wl.y));
-            const float2 t = __ffma2_rn(pc.nbeta, M, rinv);
-            e_c = __fmul2_rn(qq, t);
-            fc = __fmul2_rn(__fmul2_rn(qq, r2inv), __ffma2_rn(pc.beta_2_sqrtpi, E, t));
-        }
+        const float2 mp = polyx2(x, kEwaldMP2), mq = polyx2(x, kEwaldMQ2);
+        const float2 M = __fmul2_rn(mp, make_float2(rcp_approx(mq.x), rcp_approx(mq.y)));
+        const float2 wl = __fmul2_rn(r2, pc.nb2_log2e);
+        const float2 E = make_float2(ex2_approx(wl.x), ex2_approx(wl.y));
+        const float2 t = __ffma2_rn(pc.nbeta, M, rinv);
+        e_c = __fmul2_rn(nqq, t);
+        return __fmul2_rn(r2inv, __ffma2_rn(nqq, __ffma2_rn(pc.beta_2_sqrtpi, E, t), u));
     }
-    else
+    float c[2], e[2];
+    const float rr[2] = {r2.x, r2.y}, ri[2] = {rinv.x, rinv.y}, q[2] = {nqq.x, nqq.y};
+    for (int h2 = 0; h2 < 2; h2++)
     {
-        float c[2], e[2];
-        const float rr[2] = {r2.x, r2.y}, ri[2] = {rinv.x, rinv.y}, q[2] = {qq.x, qq.y};
-        for (int h2 = 0; h2 < 2; h2++)
-        {
-            const float r = rr[h2] * ri[h2];
-            const float br = pc.beta * r;
-            const float erfcv = erfcf(br);
-            c[h2] = q[h2] * ri[h2] * ri[h2] * ri[h2] * __fmaf_rn(br * 1.1283791670955126f, __expf(-br * br), erfcv);
-            e[h2] = q[h2] * erfcv * ri[h2];
-        }
-        fc = make_float2(c[0], c[1]);
-        if (ENERGY) e_c = make_float2(e[0], e[1]);
+        const float r = rr[h2] * ri[h2];
+        const float br = pc.beta * r;
+        const float erfcv = erfcf(br);
+        c[h2] = q[h2] * ri[h2] * ri[h2] * ri[h2] * __fmaf_rn(br * 1.1283791670955126f, __expf(-br * br), erfcv);
+        e[h2] = q[h2] * erfcv * ri[h2];
     }
-    if (ENERGY) e_lj = __ffma2_rn(B, r6inv, u);  // -A/r^12 + 2B/r^6 = -12 E_lj
-    return __ffma2_rn(fc, kPk[kPkMinusOne], flj);
+    if (ENERGY) e_c = make_float2(e[0], e[1]);
+    return __fadd2_rn(__fmul2_rn(u, r2inv), make_float2(c[0], c[1]));
 }
 
 // A difference of two 22-bit cluster-centre coordinates, wrapped to
@@ -183,45 +178,33 @@ __device__ __forceinline__ float centre_step(int qj, int qi)
 }
 
 
-__device__ __forceinline__ void cp_async(void* smem, const void* gmem, int bytes)
+// Adds to a 64-bit sum in global memory without reading it back (the compiler
+// makes a returning ATOMG of an unused atomicAdd here).
+__device__ __forceinline__ void red_add(long long* p, long long v)
 {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
-    if (bytes == 16)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem));
-    else if (bytes == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(gmem));
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gmem));
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
-__device__ __forceinline__ void cp_async_wait_prior() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// Sums eight per-lane values over the warp: after three halving exchanges
-// (lane bit 4, 3, 2 picks the half it keeps) and two full ones, lanes
-// 4v..4v+3 hold the total of value v.  Nine shuffles instead of forty.
-template <typename T>
-__device__ __forceinline__ T reduce_scatter8(const T (&v)[8], int lane)
+// Sums eight per-lane FP32 values over the warp in FP64: lanes 4r..4r+3
+// return the total of v[r].  The values are transposed through shared memory
+// (rows padded to 36 floats, so that the lanes' 16-byte reads fall on
+// different banks): lane 4r + k adds eight lanes' share of row r, and two
+// exchanges join the four parts.  33 instructions, where the same sum as
+// int64 values by shuffles takes about 110.  buf: 8 * kSumRow floats.
+constexpr int kSumRow = 36;
+__device__ __forceinline__ double lane_totals8(float* buf, const float (&v)[8], int lane)
 {
-    const bool h4 = (lane & 16) != 0, h3 = (lane & 8) != 0, h2 = (lane & 4) != 0;
-    T u[4], x[2];
+    __syncwarp();  // the buffer's last use
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-    {
-        const T send = h4 ? v[k] : v[k + 4];
-        u[k] = (h4 ? v[k + 4] : v[k]) + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
-#pragma unroll
-    for (int k = 0; k < 2; k++)
-    {
-        const T send = h3 ? u[k] : u[k + 2];
-        x[k] = (h3 ? u[k + 2] : u[k]) + __shfl_xor_sync(0xffffffffu, send, 8);
-    }
-    const T send = h2 ? x[0] : x[1];
-    T y = (h2 ? x[1] : x[0]) + __shfl_xor_sync(0xffffffffu, send, 4);
-    y += __shfl_xor_sync(0xffffffffu, y, 2);
-    y += __shfl_xor_sync(0xffffffffu, y, 1);
-    return y;
+    for (int r = 0; r < 8; r++) buf[r * kSumRow + lane] = v[r];
+    __syncwarp();
+    const float4* row = reinterpret_cast<const float4*>(buf + (lane >> 2) * kSumRow + (lane & 3) * 8);
+    const float4 x = row[0], y = row[1];
+    double s = (((double)x.x + (double)x.y) + ((double)x.z + (double)x.w)) +
+               (((double)y.x + (double)y.y) + ((double)y.z + (double)y.w));
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    return s;
 }
 
 // PME excluded-pair correction (Particle_Mesh::PME_Excluded_Force_With_Atom_Energy,
