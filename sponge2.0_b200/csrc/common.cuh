@@ -173,6 +173,7 @@ struct SysDesc
     Cell cell, rcell;
     float gl, cs2, list_radius;
     float frac_norm[3];
+    float image_bound[3];  // largest fractional extent of a cluster pair that one image serves
     int Nx, Ny, Nz, cell_begin;
     int cl_begin, cl_cap;   // the system's fixed range of clusters
     int atom_begin, atom_count, triclinic;
@@ -331,7 +332,6 @@ struct spgnb_nl
     int* d_slot_gid = nullptr;    // the same global index, compact (-1: empty slot)
     float4* d_slot_d0 = nullptr;  // offset from the cluster centre at the build
     int2* d_slot_ex = nullptr;    // first and last entry of the atom's exclusion list
-    int* d_slot_count = nullptr;  // full-list length of each slot
     // per cluster
     int* d_cl_cell = nullptr;
     int* d_cl_sys = nullptr;

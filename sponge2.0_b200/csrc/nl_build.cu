@@ -255,7 +255,7 @@ __global__ void k_cluster_props(const float3* __restrict__ crd, int* __restrict_
                                 int2* __restrict__ slot_ex, const int* __restrict__ ex_start,
                                 const int* __restrict__ ex_list, const int* __restrict__ ex_num, int clusters_cap,
                                 const int* __restrict__ need, const int* __restrict__ ncl, int* __restrict__ tcount,
-                                int* __restrict__ slot_count, int* __restrict__ pcount)
+                                int* __restrict__ pcount)
 {
     if (counters[kCntNeed] == 0) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -271,7 +271,6 @@ __global__ void k_cluster_props(const float3* __restrict__ crd, int* __restrict_
     {
         // a cluster of the system's range that this build does not use
         slot_atom[s] = -1;
-        slot_count[s] = 0;
         pcount[s] = 0;
         if (l8 == 0) tcount[k] = 0;
     }
@@ -373,27 +372,44 @@ __device__ __forceinline__ float3 frac_to_cart(float3 f, const Cell& c)
     return make_float3(f.x * c.a11 + f.y * c.a21 + f.z * c.a31, f.y * c.a22 + f.z * c.a32, f.z * c.a33);
 }
 
-// Neighbour search, one warp per cluster, its table in a deterministic order
-// (candidate runs, then cluster index) with no sorting or atomics.
+// Neighbour search: per cluster, its neighbour clusters with exact 64-bit
+// pair masks, in a deterministic order (candidate runs, then cluster index)
+// with no sorting or atomics.
 // One-sided tables (half set): a cluster keeps only neighbour clusters
 // J >= I, so each cluster pair is searched once; the pruned half list needs
 // no more, and the exports reach the lower side through the reverse index.
 // Symmetric (two-sided) tables, every neighbour cluster lower and higher:
 // for the clusters holding a flagged atom (the soft-core kernel's perturbed
 // atoms), or all clusters (dH/dlambda).  For each candidate cluster that passes a
-// conservative sphere test, the 64 atom pairs are decided as the reference
+// conservative bounding test, the 64 atom pairs are decided as the reference
 // decides them: a pair needs the higher-index atom's cell in the stencil of
 // the lower-index atom's cell, squared distance below 4*grid_length^2 in the
 // reference's FP32 expression, and no exclusion.  The distance is first
 // evaluated from the cluster-relative offsets; only pairs within 1e-4*cs2 of
-// the threshold (or of clusters whose spheres reach half a box) are
+// the threshold (or of clusters whose pairs can need their own image) are
 // re-evaluated with the reference's exact expression, so every decision is the
 // reference's.  Exclusion lists are scanned only when the partner lies within
 // the list's [first, last] range (the reference's pre-check).  A cluster pair
 // with any listed pair becomes a table element {centre difference, neighbour
 // slot base | image flag} plus its 64-bit mask (bit a*8 + b: own slot a with
-// neighbour slot b); the per-slot partner counts come out with it.
+// neighbour slot b).
+//
+// Work split.  The candidate runs' clusters are flattened over the lanes (a
+// run holds about 15, half a warp); those that pass the bounding test queue
+// in shared memory, and four at a time are decided with one neighbour atom a
+// lane against the cluster's eight atoms, two an instruction (packed FP32x2),
+// the masks assembled by ballots: about 250 instructions for four candidates,
+// where one candidate a step with two pairs a lane took over 100 for each.
+// The kernel is bound by the instructions it issues (119 M on the 96,000-atom
+// box, 259 M before; loading a step ahead only added some): 378 us to 180
+// there, 110 to 36 on an 8,200-atom box with teams.
+// TEAM = 1: a warp takes a cluster; TEAM = 4: a block of four warps takes one,
+// each a share of its candidates, their results joined in order (boxes with
+// too few clusters to fill the chip with a warp each).
 constexpr int kSearchWarps = 4;
+constexpr int kSearchBlocks = 6;    // resident blocks per SM (5: 183 us on the 96,000-atom box, 6: 180, 7, spilling: 311)
+constexpr int kSearchQueue = 256;   // candidates that passed the bounding test, waiting for their decision
+constexpr int kSearchStage = 128;   // table elements a team's warp holds until they are joined
 constexpr float kBorderBand = 1.0e-4f;
 
 __device__ bool excluded_scan(int glo, int ghi, const int* __restrict__ ex_start, const int* __restrict__ ex_list,
@@ -406,224 +422,409 @@ __device__ bool excluded_scan(int glo, int ghi, const int* __restrict__ ex_start
     return false;
 }
 
-__global__ void __launch_bounds__(kSearchWarps * 32, 5)
-    k_search(const SysDesc* __restrict__ sys, int clusters_cap, int table_cap, const int* __restrict__ need,
-             const int* __restrict__ ncl, const int* __restrict__ run_start, const int2* __restrict__ runs,
-             const int2* __restrict__ cell_cl, const int* __restrict__ cl_cell,
-             const int* __restrict__ cl_sys, const uint4* __restrict__ cl_u, const int4* __restrict__ cl_q,
-             const float4* __restrict__ cl_c, const float4* __restrict__ slot_x0, const float4* __restrict__ slot_d0,
-             const int2* __restrict__ slot_ex,
-             const int* __restrict__ ex_start, const int* __restrict__ ex_list, const int* __restrict__ ex_num,
-             int* __restrict__ tcount, float4* __restrict__ tab, uint2* __restrict__ tmask,
-             int* __restrict__ slot_count, int* counters, const int* __restrict__ go, int half,
-             const int* __restrict__ slot_atom, const unsigned char* __restrict__ two_sided_atoms)
+// The cluster's own atoms, for its whole search.
+struct __align__(16) SearchOwn
 {
-    if (go && *go == 0) return;
-    __shared__ float4 stage_t[kSearchWarps][kChunk];
-    __shared__ uint2 stage_m[kSearchWarps][kChunk];
+    float neg[3][kClusterSize];   // offsets from the centre, negated
+    int gid[kClusterSize];        // global indices (-1: empty slot)
+};
+
+struct SearchArgs
+{
+    const SysDesc* sys;
+    int clusters_cap, table_cap;
+    const int* need;
+    const int* ncl;
+    const int* run_start;
+    const int2* runs;
+    const int2* cell_cl;
+    const int* cl_cell;
+    const int* cl_sys;
+    const uint4* cl_u;
+    const int4* cl_q;
+    const float4* cl_c;
+    const float4* slot_x0;
+    const int* slot_gid;
+    const float4* slot_d0;
+    const int2* slot_ex;
+    const int *ex_start, *ex_list, *ex_num;
+    int* tcount;
+    float4* tab;
+    uint2* tmask;
+    int* counters;
+    const int* go;
+    int half;
+    const int* slot_atom;
+    const unsigned char* two_sided_atoms;
+};
+
+// The largest index distance from atom g to its exclusion list {first, last}
+// (-1: empty, at most 2^29).
+__device__ __forceinline__ int ex_reach(int g, int2 e)
+{
+    return e.y >= e.x ? min(max(abs(e.x - g), abs(e.y - g)), 1 << 29) : -1;
+}
+
+template <int TEAM>
+__global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlocks) k_search(const SearchArgs A)
+{
+    if (A.go && *A.go == 0) return;
+    __shared__ SearchOwn own_all[kSearchWarps];
+    __shared__ int queue_all[kSearchWarps][kSearchQueue];  // surviving candidates {cluster | stencil flags << 28}
+    __shared__ float4 stage_t[TEAM > 1 ? kSearchWarps : 1][TEAM > 1 ? kSearchStage : 1];
+    __shared__ uint2 stage_m[TEAM > 1 ? kSearchWarps : 1][TEAM > 1 ? kSearchStage : 1];
+    __shared__ int team_next, team_count[kSearchWarps];
     const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
+    const int w = threadIdx.x >> 5;
+    SearchOwn& own = own_all[w];
+    int* const queue = queue_all[w];
+    const unsigned below = (1u << lane) - 1u;
+    const int e_lane = lane >> 3, b_lane = lane & 7;
     unsigned long long elements = 0, listed = 0;
 
     // clusters are taken from a counter (their tables differ in length)
     for (;;)
     {
         int c = 0;
-        if (lane == 0) c = atomicAdd(&counters[kCntSearchNext], 1);
-        c = __shfl_sync(0xffffffffu, c, 0);
-        if (c >= clusters_cap) break;
-        const int sy = cl_sys[c];
-        if (!need[sy] || c - sys[sy].cl_begin >= ncl[sy]) continue;
-        const SysDesc& p = sys[sy];
-        const int cellA = cl_cell[c];
-        const uint4 ui = cl_u[c];
-        const int4 qc = cl_q[c];
+        if (TEAM == 1)
+        {
+            if (lane == 0) c = atomicAdd(&A.counters[kCntSearchNext], 1);
+            c = __shfl_sync(0xffffffffu, c, 0);
+        }
+        else
+        {
+            __syncthreads();  // the previous cluster is done with
+            if (threadIdx.x == 0) team_next = atomicAdd(&A.counters[kCntSearchNext], 1);
+            __syncthreads();
+            c = team_next;
+        }
+        if (c >= A.clusters_cap) break;
+        const int sy = A.cl_sys[c];
+        if (!A.need[sy] || c - A.sys[sy].cl_begin >= A.ncl[sy]) continue;
+        const SysDesc& p = A.sys[sy];
+        const uint4 ui = A.cl_u[c];
+        const int4 qc = A.cl_q[c];
+        const float4 hc = A.cl_c[c];
         const float ri = __uint_as_float(ui.w);
-        const float4 hc = cl_c[c];
         const float band = kBorderBand * p.cs2;
         // one-sided table, unless the cluster holds an atom flagged for two sides
-        bool one_sided = half != 0;
-        if (one_sided && two_sided_atoms)
+        bool one_sided = A.half != 0;
+        if (one_sided && A.two_sided_atoms)
         {
-            const int sa = slot_atom[c * kClusterSize + (lane & 7)];
-            one_sided = !__any_sync(0xffffffffu, sa >= 0 && two_sided_atoms[sa]);
+            const int sa = A.slot_atom[c * kClusterSize + b_lane];
+            one_sided = !__any_sync(0xffffffffu, sa >= 0 && A.two_sided_atoms[sa]);
         }
-        // the two own atoms this lane tests (rounds h = 0, 1)
-        int ga[2];
-        float3 xa[2], da[2];
-        int2 ea[2];
-        for (int h = 0; h < 2; h++)
+        unsigned own_bits;
+        int reach;  // of the cluster's exclusion lists
         {
-            const int a = h * 4 + (lane >> 3);
-            const float4 x = slot_x0[c * kClusterSize + a];
-            const float4 d = slot_d0[c * kClusterSize + a];
-            ga[h] = __float_as_int(x.w);
-            xa[h] = make_float3(x.x, x.y, x.z);
-            da[h] = make_float3(d.x, d.y, d.z);
-            ea[h] = slot_ex[c * kClusterSize + a];
-        }
-        unsigned row_count = 0;  // lanes 0-7: partners of own slot `lane`
-        int written = 0, staged = 0;
-        float4* __restrict__ my_tab = tab + (size_t)c * table_cap;
-        uint2* __restrict__ my_mask = tmask + (size_t)c * table_cap;
-        auto flush = [&](int count) {
-            const int k = written + lane;
-            if (lane < count && k < table_cap)
+            const int s = c * kClusterSize + b_lane;
+            const int g = A.slot_gid[s];
+            own_bits = __ballot_sync(0xffffffffu, g >= 0) & 0xffu;
+            reach = __reduce_max_sync(0xffffffffu, ex_reach(g, A.slot_ex[s]));
+            if (lane < kClusterSize)
             {
-                my_tab[k] = stage_t[wib][lane];
-                my_mask[k] = stage_m[wib][lane];
+                const float4 d = A.slot_d0[s];
+                own.neg[0][lane] = -d.x;
+                own.neg[1][lane] = -d.y;
+                own.neg[2][lane] = -d.z;
+                own.gid[lane] = g;
             }
-            if (lane == 0 && written + count > table_cap) atomicOr(&counters[kCntOverflow], kOvfPairs);
-            written = min(written + count, table_cap);
             __syncwarp();
+        }
+        const Cell qcell = p.qcell;
+        const float2 ncs2 = make_float2(-p.cs2, -p.cs2);
+        const bool all_safe = p.all_safe != 0;
+        float4* __restrict__ my_tab = A.tab + (size_t)c * A.table_cap;
+        uint2* __restrict__ my_mask = A.tmask + (size_t)c * A.table_cap;
+        const int r0 = A.run_start[A.cl_cell[c]], r1 = A.run_start[A.cl_cell[c] + 1];
+
+        // lane's run of the batch from r: its clusters' first id and number
+        auto load_run = [&](int r, int& first, int& n, int& flags) {
+            first = n = flags = 0;
+            if (r < r1)
+            {
+                const int2 run = A.runs[r];
+                flags = run.x & (3 << 28);
+                first = A.cell_cl[run.x & 0x0fffffff].x;
+                if (one_sided) first = max(first, c);
+                n = max(0, A.cell_cl[run.y - 1].y - first);
+            }
         };
 
-        for (int r = run_start[cellA]; r < run_start[cellA + 1]; r++)
-        {
-            const int2 run = runs[r];
-            const bool fwd = (run.x >> 28) & 1;  // the run's cells are in stencil(cellA)
-            const bool rev = (run.x >> 29) & 1;  // cellA is in their stencils
-            int b0 = cell_cl[run.x & 0x0fffffff].x;
-            const int b1 = cell_cl[run.y - 1].y;
-            for (; b0 < b1; b0 += 32)
-            {
-                const int cj = b0 + lane;
-                bool ok = false;
-                if (cj < b1 && (!one_sided || cj >= c))
+        // The elements of candidates [lo, hi) of the flattened runs, to the
+        // table (direct) or to this warp's staging; returns their number.
+        auto search = [&](int lo, int hi, bool direct) -> int {
+            int written = 0, queued = 0;
+            // four queued candidates (fewer at the end), one neighbour atom a lane
+            auto decide = [&](int q0) {
+                const bool have = q0 + e_lane < queued;
+                const int entry = have ? queue[q0 + e_lane] : c;
+                const int cj = entry & 0x0fffffff;
+                const int slot = cj * kClusterSize + b_lane;
+                const float4 dj = A.slot_d0[slot];
+                const int gb = A.slot_gid[slot];
+                const int2 ej = A.slot_ex[slot];
+                const int4 qj = A.cl_q[cj];
+                // centre difference: minimum image of the 22-bit centres
+                const float ux = (float)(((qj.x - qc.x + 0x200000) & 0x3fffff) - 0x200000);
+                const float uy = (float)(((qj.y - qc.y + 0x200000) & 0x3fffff) - 0x200000);
+                const float uz = (float)(((qj.z - qc.z + 0x200000) & 0x3fffff) - 0x200000);
+                const float Dx = ux * qcell.a11 + uy * qcell.a21 + uz * qcell.a31;
+                const float Dy = uy * qcell.a22 + uz * qcell.a32;
+                const float Dz = uz * qcell.a33;
+                // one image per cluster pair is enough when every pair of the
+                // two clusters stays inside half a box in fractional terms, or
+                // when the images it could take beyond that are out of reach
+                bool safe = true;
+                if (!all_safe)
                 {
-                    const uint4 uj = cl_u[cj];
-                    const float3 f = frac_delta(ui, uj);
+                    const uint4 uj = A.cl_u[cj];
+                    const float3 fd = frac_delta(ui, uj);
+                    const float rr = ri + __uint_as_float(uj.w);
+                    float3 ext = make_float3(rr, rr, rr);
                     if (!p.triclinic)
                     {
-                        // bounding boxes within the list radius
-                        const float3 d = frac_to_cart(f, p.cell);
-                        const float4 hj = cl_c[cj];
-                        const float gx = fmaxf(fabsf(d.x) - (hc.x + hj.x), 0.0f);
-                        const float gy = fmaxf(fabsf(d.y) - (hc.y + hj.y), 0.0f);
-                        const float gz = fmaxf(fabsf(d.z) - (hc.z + hj.z), 0.0f);
-                        ok = gx * gx + gy * gy + gz * gz < p.list_radius * p.list_radius;
+                        const float4 hj = A.cl_c[cj];
+                        ext = make_float3(hc.x + hj.x, hc.y + hj.y, hc.z + hj.z);
+                    }
+                    safe = fabsf(fd.x) + ext.x * p.frac_norm[0] < p.image_bound[0] &&
+                           fabsf(fd.y) + ext.y * p.frac_norm[1] < p.image_bound[1] &&
+                           fabsf(fd.z) + ext.z * p.frac_norm[2] < p.image_bound[2];
+                }
+                // the pairs the stencil rule allows, bit a: own atom a
+                unsigned rule = have && gb >= 0 ? own_bits : 0u;
+                if (cj == c) rule &= ~(1u << b_lane);
+                const int flags = have ? entry >> 28 & 3 : 3;
+                if (!__all_sync(0xffffffffu, flags == 3))
+                {
+                    unsigned lower = 0;
+#pragma unroll
+                    for (int a = 0; a < kClusterSize; a++) lower |= (own.gid[a] < gb ? 1u : 0u) << a;
+                    rule &= ((flags & 1) ? lower : 0u) | ((flags & 2) ? ~lower : 0u);
+                }
+                // distances, two own atoms at a time, and how near the nearest
+                // comes to the threshold (the cheap distance only decides
+                // pairs well away from it, so its rounding does not matter)
+                const float ex = Dx + dj.x, ey = Dy + dj.y, ez = Dz + dj.z;
+                const float2 ex2 = make_float2(ex, ex), ey2 = make_float2(ey, ey), ez2 = make_float2(ez, ez);
+                unsigned hit = 0;
+                float near = 3.0e38f;
+#pragma unroll
+                for (int q = 3; q >= 0; q--)
+                {
+                    const float2 dx = __fadd2_rn(ex2, reinterpret_cast<const float2*>(own.neg[0])[q]);
+                    const float2 dy = __fadd2_rn(ey2, reinterpret_cast<const float2*>(own.neg[1])[q]);
+                    const float2 dz = __fadd2_rn(ez2, reinterpret_cast<const float2*>(own.neg[2])[q]);
+                    // d^2 - cs2: its sign bits are shifted into hit
+                    const float2 t = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, ncs2)));
+                    hit = __funnelshift_l(__float_as_uint(t.y), hit, 1);
+                    hit = __funnelshift_l(__float_as_uint(t.x), hit, 1);
+                    near = fminf(near, fminf(fabsf(t.x), fabsf(t.y)));
+                }
+                if (__any_sync(0xffffffffu, rule != 0u && (!safe || near < band)))
+                {
+                    // the reference's expression for the pairs that need it
+                    const float4 xj = A.slot_x0[slot];
+#pragma unroll 1
+                    for (int a = 0; a < kClusterSize; a++)
+                    {
+                        const float dx = ex + own.neg[0][a], dy = ey + own.neg[1][a], dz = ez + own.neg[2][a];
+                        const float d2 = dx * dx + dy * dy + dz * dz;
+                        if (((rule >> a) & 1u) && (!safe || fabsf(d2 - p.cs2) < band))
+                        {
+                            const float4 xa4 = A.slot_x0[c * kClusterSize + a];
+                            const float3 xa = make_float3(xa4.x, xa4.y, xa4.z), xb = make_float3(xj.x, xj.y, xj.z);
+                            const float e2 = own.gid[a] < gb ? ref_pair_dr2(xa, xb, p.cell, p.rcell)
+                                                             : ref_pair_dr2(xb, xa, p.cell, p.rcell);
+                            hit = e2 < p.cs2 ? hit | (1u << a) : hit & ~(1u << a);
+                        }
+                    }
+                }
+                hit &= rule;
+                // an excluded partner's index lies within the reach of one of
+                // the two atoms' lists: |ga - gb| <= the larger reach, tested
+                // for all own atoms by the smallest ga - gb + reach (unsigned)
+                const int r = max(reach, ex_reach(gb, ej));
+                unsigned nearest = 0xffffffffu;
+#pragma unroll
+                for (int a = 0; a < kClusterSize; a++) nearest = min(nearest, (unsigned)(own.gid[a] + (r - gb)));
+                if (__any_sync(0xffffffffu, hit != 0u && r >= 0 && nearest <= 2u * (unsigned)r))
+                {
+                    // the lower index's list, scanned only within its range
+#pragma unroll 1
+                    for (int a = 0; a < kClusterSize; a++)
+                    {
+                        const int ga = own.gid[a];
+                        const bool a_lo = ga < gb;
+                        const int2 e = a_lo ? A.slot_ex[c * kClusterSize + a] : ej;
+                        const int hi_g = a_lo ? gb : ga;
+                        if (((hit >> a) & 1u) && hi_g >= e.x && hi_g <= e.y &&
+                            excluded_scan(a_lo ? ga : gb, a_lo ? gb : ga, A.ex_start, A.ex_list, A.ex_num))
+                            hit &= ~(1u << a);
+                    }
+                }
+                // the four candidates' masks: byte e of ballot a is own atom a's row
+                unsigned row[kClusterSize];
+#pragma unroll
+                for (int a = 0; a < kClusterSize; a++) row[a] = __ballot_sync(0xffffffffu, hit & (1u << a));
+                const unsigned pick = e_lane | (e_lane + 4) << 4;
+                uint2 m;
+                m.x = __byte_perm(__byte_perm(row[0], row[1], pick), __byte_perm(row[2], row[3], pick), 0x5410);
+                m.y = __byte_perm(__byte_perm(row[4], row[5], pick), __byte_perm(row[6], row[7], pick), 0x5410);
+                const bool lead = b_lane == 0 && (m.x | m.y) != 0u;
+                const unsigned leads = __ballot_sync(0xffffffffu, lead);
+                const int at = written + __popc(leads & below);
+                const int cap = direct ? A.table_cap : kSearchStage;
+                if (lead && at < cap)
+                {
+                    const float4 t = make_float4(Dx, Dy, Dz, __int_as_float((cj * kClusterSize) | (safe ? 0 : (1 << 30))));
+                    if (direct)
+                    {
+                        my_tab[at] = t;
+                        my_mask[at] = m;
                     }
                     else
                     {
-                        const float rsum = ri + __uint_as_float(uj.w) + p.list_radius;
-                        for (int im = 0; im < 27 && !ok; im++)
-                        {
-                            const float3 fi = make_float3(f.x + (float)(im / 9 - 1), f.y + (float)((im / 3) % 3 - 1),
-                                                          f.z + (float)(im % 3 - 1));
-                            const float3 d = frac_to_cart(fi, p.cell);
-                            ok = d.x * d.x + d.y * d.y + d.z * d.z < rsum * rsum;
-                        }
+                        stage_t[TEAM > 1 ? w : 0][TEAM > 1 ? at : 0] = t;
+                        stage_m[TEAM > 1 ? w : 0][TEAM > 1 ? at : 0] = m;
                     }
+                    listed += __popc(m.x) + __popc(m.y);
                 }
-                unsigned surv = __ballot_sync(0xffffffffu, ok);
-                while (surv)
+                written += __popc(leads);
+            };
+            // all but the last `left` queued candidates, which move to the front
+            auto work = [&](int left) {
+                __syncwarp();
+                const int end = queued - left;
+                for (int q0 = 0; q0 < end; q0 += 4) decide(q0);
+                const int keep = lane < left ? queue[end + lane] : 0;
+                __syncwarp();
+                if (lane < left) queue[lane] = keep;
+                queued = left;
+                __syncwarp();
+            };
+            int off = 0;
+            for (int rb = r0; rb < r1 && off < hi; rb += 32)
+            {
+                int first, n, flags;
+                load_run(rb + lane, first, n, flags);
+                int incl = n;
+                for (int o = 1; o < 32; o <<= 1)
                 {
-                    const int cjs = b0 + __ffs(surv) - 1;
-                    surv &= surv - 1;
-                    const int b = lane & 7;
-                    const float4 xj = slot_x0[cjs * kClusterSize + b];
-                    const float4 dj = slot_d0[cjs * kClusterSize + b];
-                    const int2 ej = slot_ex[cjs * kClusterSize + b];
-                    const int gb = __float_as_int(xj.w);
-                    const float3 xb = make_float3(xj.x, xj.y, xj.z);
-                    // centre difference: minimum image of the 22-bit centres
-                    const uint4 uj = cl_u[cjs];
-                    const int4 qj = cl_q[cjs];
-                    const float ux = (float)(((qj.x - qc.x + 0x200000) & 0x3fffff) - 0x200000);
-                    const float uy = (float)(((qj.y - qc.y + 0x200000) & 0x3fffff) - 0x200000);
-                    const float uz = (float)(((qj.z - qc.z + 0x200000) & 0x3fffff) - 0x200000);
-                    const float Dx = ux * p.qcell.a11 + uy * p.qcell.a21 + uz * p.qcell.a31;
-                    const float Dy = uy * p.qcell.a22 + uz * p.qcell.a32;
-                    const float Dz = uz * p.qcell.a33;
-                    // one image per cluster pair is enough when every pair of the
-                    // two spheres stays inside half a box in fractional terms
-                    bool safe = true;
-                    if (!p.all_safe)
-                    {
-                        const float3 fd = frac_delta(ui, uj);
-                        const float rr = ri + __uint_as_float(uj.w);
-                        safe = fabsf(fd.x) + rr * p.frac_norm[0] < 0.49f && fabsf(fd.y) + rr * p.frac_norm[1] < 0.49f &&
-                               fabsf(fd.z) + rr * p.frac_norm[2] < 0.49f;
-                    }
-                    unsigned bits[2];
-                    // both rounds' distances first, then one vote for the border
-                    // cases (the cheap distance only decides pairs well away
-                    // from the threshold, so its rounding does not matter)
-                    const float ex = Dx + dj.x, ey = Dy + dj.y, ez = Dz + dj.z;
-                    const bool gb_ok = gb >= 0, self = cjs == c;
-                    bool in_h[2], border_h[2], rule_h[2];
-#pragma unroll
-                    for (int h = 0; h < 2; h++)
-                    {
-                        const int a = h * 4 + (lane >> 3);
-                        const bool a_lo = ga[h] < gb;
-                        rule_h[h] = ga[h] >= 0 && gb_ok && (!self || b != a) && (a_lo ? fwd : rev);
-                        const float dx = ex - da[h].x, dy = ey - da[h].y, dz = ez - da[h].z;
-                        const float d2 = dx * dx + dy * dy + dz * dz;
-                        border_h[h] = rule_h[h] && (!safe || fabsf(d2 - p.cs2) < band);
-                        in_h[h] = d2 < p.cs2;
-                    }
-                    if (__any_sync(0xffffffffu, border_h[0] || border_h[1]))
-                    {
-#pragma unroll
-                        for (int h = 0; h < 2; h++)
-                            if (border_h[h])
-                            {
-                                const float e2 = ga[h] < gb ? ref_pair_dr2(xa[h], xb, p.cell, p.rcell)
-                                                            : ref_pair_dr2(xb, xa[h], p.cell, p.rcell);
-                                in_h[h] = e2 < p.cs2;
-                            }
-                    }
-#pragma unroll
-                    for (int h = 0; h < 2; h++)
-                    {
-                        const bool a_lo = ga[h] < gb;
-                        bool in = in_h[h] && rule_h[h];
-                        if (in)
-                        {
-                            // the lower index's exclusion list, scanned only within its range
-                            const int2 e = a_lo ? ea[h] : ej;
-                            const int glo = a_lo ? ga[h] : gb, ghi = a_lo ? gb : ga[h];
-                            if (ghi >= e.x && ghi <= e.y) in = !excluded_scan(glo, ghi, ex_start, ex_list, ex_num);
-                        }
-                        bits[h] = __ballot_sync(0xffffffffu, in);
-                    }
-                    if (bits[0] | bits[1])
-                    {
-                        const unsigned long long m = ((unsigned long long)bits[1] << 32) | bits[0];
-                        if (written + staged < table_cap && lane < 8) row_count += __popc((unsigned)(m >> (8 * lane)) & 0xffu);
-                        if (lane == 0)
-                        {
-                            stage_t[wib][staged] = make_float4(Dx, Dy, Dz,
-                                                               __int_as_float((cjs * kClusterSize) | (safe ? 0 : (1 << 30))));
-                            stage_m[wib][staged] = make_uint2(bits[0], bits[1]);
-                        }
-                        staged++;
-                        __syncwarp();
-                        if (staged == kChunk)
-                        {
-                            flush(kChunk);
-                            staged = 0;
-                        }
-                    }
+                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
                 }
+                const int total = __shfl_sync(0xffffffffu, incl, 31);
+                const int base = first - (incl - n);
+                const int t1 = min(hi - off, total);
+                for (int t0 = max(lo - off, 0); t0 < t1; t0 += 32)
+                {
+                    // the run candidate t falls into: the number of runs that end at or before it
+                    const int t = t0 + lane;
+                    int k = 0;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1)
+                        if (__shfl_sync(0xffffffffu, incl, k + o - 1) <= t) k += o;
+                    k = min(k, 31);
+                    const int cj = __shfl_sync(0xffffffffu, base, k) + t;
+                    const int fl = __shfl_sync(0xffffffffu, flags, k);
+                    bool ok = false;
+                    if (t < t1)
+                    {
+                        const uint4 uj = A.cl_u[cj];
+                        const float3 f = frac_delta(ui, uj);
+                        if (!p.triclinic)
+                        {
+                            // bounding boxes within the list radius
+                            const float3 d = frac_to_cart(f, p.cell);
+                            const float4 hj = A.cl_c[cj];
+                            const float gx = fmaxf(fabsf(d.x) - (hc.x + hj.x), 0.0f);
+                            const float gy = fmaxf(fabsf(d.y) - (hc.y + hj.y), 0.0f);
+                            const float gz = fmaxf(fabsf(d.z) - (hc.z + hj.z), 0.0f);
+                            ok = gx * gx + gy * gy + gz * gz < p.list_radius * p.list_radius;
+                        }
+                        else
+                        {
+                            const float rsum = ri + __uint_as_float(uj.w) + p.list_radius;
+                            for (int im = 0; im < 27 && !ok; im++)
+                            {
+                                const float3 fi = make_float3(f.x + (float)(im / 9 - 1), f.y + (float)((im / 3) % 3 - 1),
+                                                              f.z + (float)(im % 3 - 1));
+                                const float3 d = frac_to_cart(fi, p.cell);
+                                ok = d.x * d.x + d.y * d.y + d.z * d.z < rsum * rsum;
+                            }
+                        }
+                    }
+                    const unsigned surv = __ballot_sync(0xffffffffu, ok);
+                    if (ok) queue[queued + __popc(surv & below)] = cj | fl;
+                    queued += __popc(surv);
+                    if (queued > kSearchQueue - 32) work(queued & 3);
+                }
+                off += total;
+            }
+            work(0);
+            return written;
+        };
+
+        if (TEAM == 1)
+        {
+            const int written = search(0, 0x7fffffff, true);
+            if (lane == 0)
+            {
+                if (written > A.table_cap) atomicOr(&A.counters[kCntOverflow], kOvfPairs);
+                A.tcount[c] = min(written, A.table_cap);
+                elements += (unsigned long long)min(written, A.table_cap);
             }
         }
-        if (staged > 0) flush(staged);
-        if (lane < 8) slot_count[c * kClusterSize + lane] = (int)row_count;
-        unsigned long long words = lane < 8 ? row_count : 0u;
-        for (int o = 16; o > 0; o >>= 1) words += __shfl_xor_sync(0xffffffffu, words, o);
-        if (lane == 0)
+        else
         {
-            tcount[c] = written;
-            elements += (unsigned long long)written;
-            listed += words;
+            // the team's shares of the candidates, in order
+            int all = 0;
+            for (int rb = r0; rb < r1; rb += 32)
+            {
+                int first, n, flags;
+                load_run(rb + lane, first, n, flags);
+                all += __reduce_add_sync(0xffffffffu, n);
+            }
+            const unsigned long long before = listed;
+            const int count = search((int)((long long)all * w / TEAM), (int)((long long)all * (w + 1) / TEAM), false);
+            if (lane == 0) team_count[w] = count;
+            __syncthreads();
+            int start = 0, sum = 0, most = 0;
+#pragma unroll
+            for (int v = 0; v < TEAM; v++)
+            {
+                const int k = team_count[v];
+                if (v < w) start += k;
+                sum += k;
+                most = max(most, k);
+            }
+            if (most > kSearchStage)
+            {
+                // a share that does not fit its staging: one warp for all
+                listed = before;
+                if (w == 0) sum = search(0, 0x7fffffff, true);
+            }
+            else
+                for (int k = lane; k < count; k += 32)
+                    if (start + k < A.table_cap)
+                    {
+                        my_tab[start + k] = stage_t[w][TEAM > 1 ? k : 0];
+                        my_mask[start + k] = stage_m[w][TEAM > 1 ? k : 0];
+                    }
+            if (threadIdx.x == 0)
+            {
+                if (sum > A.table_cap) atomicOr(&A.counters[kCntOverflow], kOvfPairs);
+                A.tcount[c] = min(sum, A.table_cap);
+                elements += (unsigned long long)min(sum, A.table_cap);
+            }
         }
     }
+    for (int o = 16; o > 0; o >>= 1) listed += __shfl_xor_sync(0xffffffffu, listed, o);
     if (lane == 0)
     {
-        if (elements) atomicAdd((unsigned long long*)&counters[kCntEntries], elements);
-        if (listed) atomicAdd((unsigned long long*)&counters[kCntWords], listed);
+        if (elements) atomicAdd((unsigned long long*)&A.counters[kCntEntries], elements);
+        if (listed) atomicAdd((unsigned long long*)&A.counters[kCntWords], listed);
     }
 }
 
@@ -987,6 +1188,52 @@ __global__ void k_init_atom_groups(int n, spgnb_atom_group* nl, int* temp, int m
 
 // --------------------------------------------------------------- host side
 
+// The search of the list's clusters (go: the device flag that lets it run,
+// null: always).  A block of four warps per cluster while the chip has room
+// for that many blocks (eight a SM), else a warp per cluster: with fewer
+// clusters than the chip has warps, one warp's walk over a cluster's
+// candidates is the kernel's time.
+int launch_search(const spgnb_nl* nl, const int* need, const int* ex_start, const int* ex_list, const int* ex_num,
+                  const int* go, int half, const unsigned char* two_sided, cudaStream_t s)
+{
+    SearchArgs a;
+    a.sys = nl->d_sys;
+    a.clusters_cap = nl->clusters_cap;
+    a.table_cap = nl->table_cap;
+    a.need = need;
+    a.ncl = nl->d_ncl;
+    a.run_start = nl->d_run_start;
+    a.runs = nl->d_runs;
+    a.cell_cl = nl->d_cell_cl;
+    a.cl_cell = nl->d_cl_cell;
+    a.cl_sys = nl->d_cl_sys;
+    a.cl_u = nl->d_cl_u;
+    a.cl_q = nl->d_cl_q;
+    a.cl_c = nl->d_cl_c;
+    a.slot_x0 = nl->d_slot_x0;
+    a.slot_gid = nl->d_slot_gid;
+    a.slot_d0 = nl->d_slot_d0;
+    a.slot_ex = nl->d_slot_ex;
+    a.ex_start = ex_start;
+    a.ex_list = ex_list;
+    a.ex_num = ex_num;
+    a.tcount = nl->d_tcount;
+    a.tab = nl->d_tab;
+    a.tmask = nl->d_tmask;
+    a.counters = nl->d_counters;
+    a.go = go;
+    a.half = half;
+    a.slot_atom = nl->d_slot_atom;
+    a.two_sided_atoms = two_sided;
+    const int ccap = nl->clusters_cap, sms = num_sms();
+    if (ccap <= sms * 16)
+        k_search<4><<<std::max(1, std::min(ccap, sms * 8)), kSearchWarps * 32, 0, s>>>(a);
+    else
+        k_search<1><<<std::max(1, std::min((ccap + kSearchWarps - 1) / kSearchWarps, sms * 8)), kSearchWarps * 32, 0, s>>>(a);
+    SPGNB_CHECK_LAUNCH("k_search");
+    return SPGNB_OK;
+}
+
 void grid_dims(const spgnb_ltmatrix3& cell, float cutoff, float skin, int dims[3], float* gl)
 {
     const float g = 0.5f * (cutoff + skin);
@@ -1113,7 +1360,6 @@ void free_nl(spgnb_nl* nl)
     dfree(nl->d_slot_gid);
     dfree(nl->d_slot_d0);
     dfree(nl->d_slot_ex);
-    dfree(nl->d_slot_count);
     dfree(nl->d_cl_cell);
     dfree(nl->d_cl_sys);
     dfree(nl->d_cl_u);
@@ -1209,6 +1455,11 @@ SysDesc make_desc(const SysHost& sh, float skin_permit)
     d.frac_norm[0] = sqrtf(d.rcell.a11 * d.rcell.a11 + d.rcell.a21 * d.rcell.a21 + d.rcell.a31 * d.rcell.a31);
     d.frac_norm[1] = sqrtf(d.rcell.a22 * d.rcell.a22 + d.rcell.a32 * d.rcell.a32);
     d.frac_norm[2] = fabsf(d.rcell.a33);
+    // a pair beyond half a box in a fractional coordinate f has another image
+    // at 1 - f; past this bound on f that image could come within the list
+    // radius, and the pair needs its own
+    for (int k = 0; k < 3; k++)
+        d.image_bound[k] = fmaxf(0.49f, 1.0f - 1e-4f - (d.list_radius + 0.01f) * d.frac_norm[k]);
     d.Nx = sh.dims[0];
     d.Ny = sh.dims[1];
     d.Nz = sh.dims[2];
@@ -1291,8 +1542,6 @@ int alloc_nl(spgnb_nl* nl)
     if ((st = dalloc(&nl->d_slot_d0, slots))) return st;
     SPGNB_CUDA(cudaMemset(nl->d_slot_d0, 0, sizeof(float4) * slots));
     if ((st = dalloc(&nl->d_slot_ex, slots))) return st;
-    if ((st = dalloc(&nl->d_slot_count, slots))) return st;
-    SPGNB_CUDA(cudaMemset(nl->d_slot_count, 0, sizeof(int) * slots));
     if ((st = dalloc(&nl->d_pcount, slots))) return st;
     if ((st = dalloc(&nl->d_facc, 3 * (size_t)slots))) return st;
     SPGNB_CUDA(cudaMemset(nl->d_facc, 0, sizeof(long long) * 3 * (size_t)slots));
@@ -1517,7 +1766,6 @@ int nl_retire(spgnb_nl* nl, int id, cudaStream_t s)
     SPGNB_CUDA(cudaMemsetAsync(nl->d_cell_cursor + sh.cell_begin, 0, sizeof(int) * (G + 1), s));
     if ((st = fill_int(nl->d_cl_sys + sh.cl_begin, sh.cl_cap, nl->S, s))) return st;
     SPGNB_CUDA(cudaMemsetAsync(nl->d_slot_atom + slot0, 0xff, sizeof(int) * nslots, s));
-    SPGNB_CUDA(cudaMemsetAsync(nl->d_slot_count + slot0, 0, sizeof(int) * nslots, s));
     SPGNB_CUDA(cudaMemsetAsync(nl->d_pcount + slot0, 0, sizeof(int) * nslots, s));
     SPGNB_CUDA(cudaMemsetAsync(nl->d_tcount + sh.cl_begin, 0, sizeof(int) * sh.cl_cap, s));
     k_sys_flags<<<1, 1, 0, s>>>(id, 0, nl->d_live, nl->d_need, nl->d_prune, nl->d_ncl);
@@ -1546,7 +1794,7 @@ size_t nl_device_bytes(const spgnb_nl* nl)
     const size_t n = nl->n_cap, G = nl->G, S = nl->S + 1, C = nl->clusters_cap, slots = C * kClusterSize;
     size_t b = 0;
     b += n * (4 + 4 + 4 + 16 + 4);                                   // atom system, cell, shift, wrapped, slot
-    b += slots * (4 + 4 + 16 + 4 + 16 + 8 + 4 + 4 + 24 + 64 + 16);   // per-slot arrays (with the int64 staging)
+    b += slots * (4 + 4 + 16 + 4 + 16 + 8 + 4 + 24 + 64 + 16);   // per-slot arrays (with the int64 staging)
     b += C * (size_t)nl->list_cap * 4;                               // pruned lists
     b += C * (4 + 4 + 16 + 16 + 16 + 4) + 16;                        // per-cluster arrays
     b += C * (size_t)nl->table_cap * (16 + 8);                       // neighbour tables
@@ -1694,16 +1942,11 @@ int nl_queue_build_body(spgnb_nl* nl, int n, const float3* d_crd, const int* d_a
     k_cluster_props<<<(slots_cap + 255) / 256, 256, 0, s>>>(
         d_crd, nl->d_slot_atom, nl->d_atom_shift, d_atom_local, nl->d_cl_sys, nl->d_sys, nl->d_counters, nl->d_cl_u,
         nl->d_cl_q, nl->d_cl_c, nl->d_slot_x0, nl->d_slot_gid, nl->d_slot_d0, nl->d_slot_ex, ex_start, ex_list, ex_num,
-        ccap, nl->d_need, nl->d_ncl, nl->d_tcount, nl->d_slot_count, nl->d_pcount);
+        ccap, nl->d_need, nl->d_ncl, nl->d_tcount, nl->d_pcount);
     SPGNB_CHECK_LAUNCH("k_cluster_props");
-    // one resident wave (five blocks per SM)
-    const int search_blocks = std::max(1, std::min((ccap + kSearchWarps - 1) / kSearchWarps, sms * 5));
-    k_search<<<search_blocks, kSearchWarps * 32, 0, s>>>(
-        nl->d_sys, ccap, nl->table_cap, nl->d_need, nl->d_ncl, nl->d_run_start, nl->d_runs, nl->d_cell_cl,
-        nl->d_cl_cell, nl->d_cl_sys, nl->d_cl_u, nl->d_cl_q, nl->d_cl_c, nl->d_slot_x0, nl->d_slot_d0, nl->d_slot_ex,
-        ex_start, ex_list, ex_num, nl->d_tcount, nl->d_tab, nl->d_tmask, nl->d_slot_count, nl->d_counters,
-        nl->d_counters + kCntNeed, 1, nl->d_slot_atom, nl->two_sided_atoms);
-    SPGNB_CHECK_LAUNCH("k_search");
+    const int st_search = launch_search(nl, nl->d_need, ex_start, ex_list, ex_num, nl->d_counters + kCntNeed, 1,
+                                        nl->two_sided_atoms, s);
+    if (st_search) return st_search;
     nl->sym_built = false;
     nl->two_sided_built = nl->two_sided_atoms;
     nl->rev_built = false;
@@ -1978,16 +2221,11 @@ int research_last_build(const spgnb_nl* nl, cudaStream_t s, int half, const unsi
 {
     k_sym_begin<<<1, 1, 0, s>>>(nl->d_counters);
     SPGNB_CHECK_LAUNCH("k_sym_begin");
-    const int ccap = nl->clusters_cap;
-    const int search_blocks = std::max(1, std::min((ccap + kSearchWarps - 1) / kSearchWarps, num_sms() * 5));
     // every live system, whatever the last build flagged: a system's tables
     // are those of its own last build either way
-    k_search<<<search_blocks, kSearchWarps * 32, 0, s>>>(
-        nl->d_sys, ccap, nl->table_cap, nl->d_live, nl->d_ncl, nl->d_run_start, nl->d_runs, nl->d_cell_cl,
-        nl->d_cl_cell, nl->d_cl_sys, nl->d_cl_u, nl->d_cl_q, nl->d_cl_c, nl->d_slot_x0, nl->d_slot_d0, nl->d_slot_ex,
-        nl->ex_start_last, nl->ex_list_last, nl->ex_num_last, nl->d_tcount, nl->d_tab, nl->d_tmask, nl->d_slot_count,
-        nl->d_counters, nullptr, half, nl->d_slot_atom, flags);
-    SPGNB_CHECK_LAUNCH("k_search");
+    const int st = launch_search(nl, nl->d_live, nl->ex_start_last, nl->ex_list_last, nl->ex_num_last, nullptr, half,
+                                 flags, s);
+    if (st) return st;
     nl->rev_built = false;  // the tables' elements moved
     return SPGNB_OK;
 }
