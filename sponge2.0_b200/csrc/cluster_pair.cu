@@ -30,7 +30,9 @@ namespace spgnb
 namespace
 {
 
-constexpr int kPruneWarps = 8;
+constexpr int kPruneWarps = 4;
+constexpr int kPruneAhead = 8;                      // pruning steps whose partners are loaded together
+constexpr int kPruneStage = 384;                   // words a team's warp holds until they are joined
 constexpr int kWindow = 32;                        // list parts are padded to whole 32-word windows
 constexpr unsigned kWordSlotMask = (1u << 22) - 1u; // partner slot field of a list word
 constexpr int kWordMaskShift = 22;                  // the 8-bit atom mask
@@ -115,14 +117,24 @@ __global__ void k_pack_slots(int slots_cap, int* counters, const int* __restrict
 
 // Pruning (no reference counterpart; results unchanged).  Runs after every
 // rebuild and whenever some atom of a system moved more than buffer/2 since
-// its last one (the pack kernel checks).  One warp per cluster I walks the
+// its last one (the pack kernel checks).  For cluster I it walks the
 // elements of its neighbour table with J >= I (a table built one-sided holds
-// no others), expands the union of the eight atoms' mask rows 32 elements at
-// a time into shared memory, loads each candidate partner once, tests it
-// against all eight atoms without branches (packed FP32x2, two atoms an
-// instruction) and writes one word per partner within cutoff + buffer of any
-// of them, in table order, padded to a whole window with words whose mask is
-// empty.  The last block to finish clears the flags.
+// no others), four at a time, one neighbour atom a lane: its own-atom mask
+// bits come from the element's mask by a bit gather, it is tested against all
+// eight atoms without branches (packed FP32x2, two atoms an instruction), and
+// one word per partner within cutoff + buffer of any of them is written, in
+// table order, padded to a whole window with words whose mask is empty.
+// A chunk of 32 elements is loaded while the one before it is worked on, and
+// its partners all together: with one step's loads in flight at a time the
+// kernel waited for them (76 us on the 96,000-atom box against 57 now; four
+// steps' partners together 58).  The form before, which first compacted each
+// chunk's partners in shared memory, took 58 there, and 40 against 8 now on
+// the 1,944-atom box, where a team works on each cluster.
+// TEAM = 1: a warp takes a cluster; TEAM = 4: a block of four warps, each a
+// share of the table, their words joined in order (few clusters: one warp's
+// walk would be the kernel's time).  The last block to finish clears the
+// flags.
+template <int TEAM>
 __global__ void __launch_bounds__(kPruneWarps * 32)
     k_prune8(ForceParams p0, const ForceParams* __restrict__ fps, float buffer, int* counters, int clusters_cap,
              int table_cap, int list_cap, const int* __restrict__ cl_sys, const SysDesc* __restrict__ sys,
@@ -132,39 +144,50 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
 {
     grid_dep_wait();
     if (counters[kCntPrune] == 0) return;
-    // a chunk's candidates {partner slot | image flag, element lane | own-atom bits << 5}
-    __shared__ uint2 buf[kPruneWarps][kChunk * kClusterSize];
-    __shared__ float4 own_all[kPruneWarps][kClusterSize];
     // the cluster's atoms negated, per coordinate, as four {even, odd} float2
     __shared__ __align__(16) float nown_all[kPruneWarps][3][kClusterSize];
-    __shared__ float4 ent_all[kPruneWarps][32];  // the window's table elements (centre differences)
+    __shared__ float4 ent_all[kPruneWarps][32];  // a chunk's table elements
+    __shared__ uint2 msk_all[kPruneWarps][32];
+    __shared__ unsigned stage_all[TEAM > 1 ? kPruneWarps : 1][TEAM > 1 ? kPruneStage : 1];
+    __shared__ int team_next, team_count[kPruneWarps], team_image[kPruneWarps];
     __shared__ unsigned long long kept_total;
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
     if (threadIdx.x == 0) kept_total = 0;
     __syncthreads();
-    uint2* __restrict__ mybuf = buf[w];
-    float4* __restrict__ own = own_all[w];
-    const float2* __restrict__ nown = reinterpret_cast<const float2*>(&nown_all[w][0][0]);
-    float4* __restrict__ ent = ent_all[w];
+    float(&own)[3][kClusterSize] = nown_all[w];
+    const float2* __restrict__ nown = reinterpret_cast<const float2*>(&own[0][0]);
+    float4* ent = ent_all[w];
+    uint2* msk = msk_all[w];
     const unsigned below = (1u << lane) - 1u;
+    const int e_lane = lane >> 3, b_lane = lane & 7;
     for (;;)
     {
         int c = 0;
-        if (lane == 0) c = atomicAdd(&counters[kCntPruneNext], 1);
-        c = __shfl_sync(0xffffffffu, c, 0);
+        if (TEAM == 1)
+        {
+            if (lane == 0) c = atomicAdd(&counters[kCntPruneNext], 1);
+            c = __shfl_sync(0xffffffffu, c, 0);
+        }
+        else
+        {
+            __syncthreads();  // the previous cluster is done with
+            if (threadIdx.x == 0) team_next = atomicAdd(&counters[kCntPruneNext], 1);
+            __syncthreads();
+            c = team_next;
+        }
         if (c >= clusters_cap) break;
         const int sy = cl_sys[c];
         if (!prune[sy]) continue;
         const int s0 = c * kClusterSize;
+        __syncwarp();
         if (lane < kClusterSize)
         {
             const float4 pl = pos[s0 + lane];
-            own[lane] = pl;
-            nown_all[w][0][lane] = -pl.x;
-            nown_all[w][1][lane] = -pl.y;
-            nown_all[w][2][lane] = -pl.z;
-            pref[s0 + lane] = pl;
+            own[0][lane] = -pl.x;
+            own[1][lane] = -pl.y;
+            own[2][lane] = -pl.z;
+            if (TEAM == 1 || w == 0) pref[s0 + lane] = pl;
         }
         __syncwarp();
         const SysDesc& D = sys[sy];
@@ -172,126 +195,153 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
         const ForceParams P = fps ? fps[sy] : p0;
         const float rp = sqrtf(P.rc2) + buffer + 1e-3f;
         const float rp2 = buffer > 0.0f ? rp * rp : 3.0e38f;
-        const int T = tcount[c];
+        const float2 nrp2 = f2(-rp2);
         const float4* __restrict__ tb = tab + (size_t)c * table_cap;
         const uint2* __restrict__ tm = tmask + (size_t)c * table_cap;
         unsigned* __restrict__ wc = words + (size_t)c * list_cap;
         const int usable = list_cap - kWindow;  // room left for the padding
-        int kh = 0;
         unsigned any_image = 0;
-        for (int t0 = 0; t0 < T; t0 += 32)
-        {
-            const int t = t0 + lane;
-            uint2 mm = make_uint2(0u, 0u);
-            float4 e = make_float4(0, 0, 0, 0);
-            if (t < T)
-            {
-                e = tb[t];
-                mm = tm[t];
-                // clusters below I hold the other side of its pairs
-                if (((__float_as_int(e.w) & 0x3fffffff) >> 3) < c) mm = make_uint2(0u, 0u);
-            }
-            // partners of any of the eight atoms
-            unsigned u = mm.x | mm.y;
-            u |= u >> 16;
-            u |= u >> 8;
-            const unsigned row = u & 0xffu;
-            const int cnt = __popc(row);
-            int incl = cnt;
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            const int eb = __float_as_int(e.w);
-            const unsigned flag = (eb & (1 << 30)) ? 0x80000000u : 0u;
-            const unsigned base = (unsigned)(eb & 0x3fffffff) | flag;
-            int k = incl - cnt;
-            // own atom a pairs with neighbour slot b when bit 8a + b is set;
-            // transposed, byte b holds neighbour b's own-atom bits
-            const unsigned long long tm8 = transpose8x8(((unsigned long long)mm.y << 32) | mm.x);
-            ent[lane] = e;
-#pragma unroll
-            for (int b = 0; b < kClusterSize; b++)
-                if ((row >> b) & 1u)
+
+        // The words of table elements [lo, hi), to `out` (room of them);
+        // returns their number.
+        auto walk = [&](int lo, int hi, unsigned* out, int room) -> int {
+            int kept = 0;
+            auto element = [&](int t, float4& e, uint2& m) {
+                e = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(s0));
+                m = make_uint2(0u, 0u);
+                if (t < hi)
                 {
-                    const unsigned am = (unsigned)(tm8 >> (8 * b)) & 0xffu;
-                    mybuf[k++] = make_uint2(base + b, (unsigned)lane | (am << 5));
+                    e = tb[t];
+                    m = tm[t];
+                    // clusters below I hold the other side of its pairs
+                    if ((__float_as_int(e.w) & 0x3fffffff) < s0) m = make_uint2(0u, 0u);
                 }
-            __syncwarp();
-            // a lane's candidate of an iteration: its record and own-atom
-            // bits; the partner's position is loaded an iteration ahead
-            auto candidate = [&](int q, uint2& wv, unsigned& am, float4& pj) {
-                wv = mybuf[q < total ? q : 0];
-                am = q < total ? (wv.y >> 5) & 0xffu : 0u;
-                pj = make_float4(0, 0, 0, 0);
-                if (am) pj = pos[wv.x & 0x7fffffffu];
             };
-            uint2 wv_next;
-            unsigned am_next;
-            float4 pj_next;
-            candidate(lane, wv_next, am_next, pj_next);
-            for (int q0 = 0; q0 < total; q0 += 32)
+            float4 en;
+            uint2 mn;
+            element(lo + lane, en, mn);
+            for (int t0 = lo; t0 < hi; t0 += 32)
             {
-                const uint2 wv = wv_next;
-                const unsigned am = am_next;
-                const float4 pj = pj_next;
-                if (q0 + 32 < total) candidate(q0 + 32 + lane, wv_next, am_next, pj_next);
-                // the element's centre difference, staged by the lane that read it
-                const float4 es = ent[wv.y & 31u];
-                const float ex = es.x, ey = es.y, ez = es.z;
-                const int js = (int)(wv.x & 0x7fffffffu);
-                const bool img = (wv.x & 0x80000000u) != 0;
-                // bit a: own atom a lies within the pruning radius of the
-                // partner.  All eight are tested without branches; the
-                // minimum-image path (small boxes) only when a lane needs it.
-                unsigned hit = 0;
-                if (!__any_sync(0xffffffffu, img && am != 0u))
-                {
-                    // the partner in the cluster's frame, then two own atoms
-                    // at a time in packed FP32x2
-                    const float2 cx = make_float2(ex + pj.x, ex + pj.x), cy = make_float2(ey + pj.y, ey + pj.y),
-                                 cz = make_float2(ez + pj.z, ez + pj.z);
-#pragma unroll
-                    for (int p = 0; p < 4; p++)
-                    {
-                        const float2 dx = __fadd2_rn(cx, nown[p]), dy = __fadd2_rn(cy, nown[4 + p]),
-                                     dz = __fadd2_rn(cz, nown[8 + p]);
-                        const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-                        hit |= ((r2.x < rp2 ? 1u : 0u) | (r2.y < rp2 ? 2u : 0u)) << (2 * p);
-                    }
-                }
-                else
-                {
+                __syncwarp();
+                ent[lane] = en;
+                msk[lane] = mn;
+                __syncwarp();
+                element(t0 + 32 + lane, en, mn);
+                const int quads = min(8, (hi - t0 + 3) / 4);
 #pragma unroll 1
-                    for (int a = 0; a < kClusterSize; a++)
+                for (int g = 0; g < quads; g += kPruneAhead)
+                {
+                    float4 pjs[kPruneAhead];
+#pragma unroll
+                    for (int k = 0; k < kPruneAhead; k++)
+                        pjs[k] = pos[(__float_as_int(ent[4 * (g + k) + e_lane].w) & 0x3fffffff) + b_lane];
+#pragma unroll
+                    for (int k = 0; k < kPruneAhead; k++)
                     {
-                        const float3 d = pair_offset(ex, ey, ez, own[a], pj, img, D);
-                        if (__fmaf_rn(d.z, d.z, __fmaf_rn(d.y, d.y, d.x * d.x)) < rp2) hit |= 1u << a;
+                        if (g + k >= quads) break;
+                        const float4 e = ent[4 * (g + k) + e_lane], pj = pjs[k];
+                        const uint2 m = msk[4 * (g + k) + e_lane];
+                        // the partner's own-atom bits: bit 8a + b of the element's
+                        // mask for a = 0..7 (a multiplication gathers four bits)
+                        const unsigned am = (((m.x >> b_lane) & 0x01010101u) * 0x01020408u) >> 24 |
+                                            ((((m.y >> b_lane) & 0x01010101u) * 0x01020408u) >> 24) << 4;
+                        const int eb = __float_as_int(e.w);
+                        const unsigned js = (unsigned)(eb & 0x3fffffff) + b_lane;
+                        const bool img = (eb & (1 << 30)) != 0;
+                        // bit a: own atom a lies within the pruning radius of
+                        // the partner; the minimum-image path (small boxes)
+                        // only when a lane needs it
+                        unsigned hit = 0;
+                        if (!__any_sync(0xffffffffu, img && am != 0u))
+                        {
+                            const float2 cx = make_float2(e.x + pj.x, e.x + pj.x),
+                                         cy = make_float2(e.y + pj.y, e.y + pj.y),
+                                         cz = make_float2(e.z + pj.z, e.z + pj.z);
+#pragma unroll
+                            for (int p = 3; p >= 0; p--)
+                            {
+                                // r^2 - rp^2: its sign bits are shifted into hit
+                                const float2 dx = __fadd2_rn(cx, nown[p]), dy = __fadd2_rn(cy, nown[4 + p]),
+                                             dz = __fadd2_rn(cz, nown[8 + p]);
+                                const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, nrp2)));
+                                hit = __funnelshift_l(__float_as_uint(r2.y), hit, 1);
+                                hit = __funnelshift_l(__float_as_uint(r2.x), hit, 1);
+                            }
+                        }
+                        else
+                        {
+#pragma unroll 1
+                            for (int a = 0; a < kClusterSize; a++)
+                            {
+                                const float4 pi = make_float4(-own[0][a], -own[1][a], -own[2][a], 0.0f);
+                                const float3 d = pair_offset(e.x, e.y, e.z, pi, pj, img, D);
+                                if (__fmaf_rn(d.z, d.z, __fmaf_rn(d.y, d.y, d.x * d.x)) < rp2) hit |= 1u << a;
+                            }
+                        }
+                        hit &= am;
+                        // partners in later clusters pair with every atom they
+                        // reach; within the cluster only the pairs a < b
+                        if ((js >> 3) == (unsigned)c) hit &= (1u << b_lane) - 1u;
+                        const unsigned mh = __ballot_sync(0xffffffffu, hit != 0u);
+                        const int at = kept + __popc(mh & below);
+                        if (hit && at < room)
+                            out[at] = (js - slot0) | (img ? kWordImage : 0u) | (hit << kWordMaskShift);
+                        any_image |= img && hit != 0u ? 1u : 0u;
+                        kept += __popc(mh);
                     }
                 }
-                hit &= am;
-                // partners in later clusters pair with every atom they reach;
-                // within the cluster only the pairs a < b
-                if ((js >> 3) == c) hit &= (1u << (js & 7)) - 1u;
-                const unsigned wb = ((unsigned)js - slot0) | (img ? kWordImage : 0u);
-                const unsigned mh = __ballot_sync(0xffffffffu, hit != 0u);
-                const int kh_next = kh + __popc(mh);
-                if (kh_next <= usable)
-                {
-                    if (hit) wc[kh + __popc(mh & below)] = wb | (hit << kWordMaskShift);
-                    any_image |= __any_sync(0xffffffffu, img && hit != 0u);
-                }
-                else if (lane == 0)
-                    atomicOr(&counters[kCntOverflow], kOvfWords);
-                kh = kh_next;
             }
-            __syncwarp();
+            return kept;
+        };
+
+        const int T = tcount[c];
+        int kh;
+        if (TEAM == 1)
+        {
+            kh = walk(0, T, wc, usable);
+            any_image = __any_sync(0xffffffffu, any_image);
+        }
+        else
+        {
+            unsigned* stage = stage_all[TEAM > 1 ? w : 0];
+            const int quads = (T + 3) / 4;
+            const int kept = walk(4 * (quads * w / TEAM), min(T, 4 * (quads * (w + 1) / TEAM)), stage, kPruneStage);
+            any_image = __any_sync(0xffffffffu, any_image);
+            if (lane == 0)
+            {
+                team_count[w] = kept;
+                team_image[w] = (int)any_image;
+            }
+            __syncthreads();
+            int start = 0, most = 0;
+            kh = 0;
+            any_image = 0;
+#pragma unroll
+            for (int v = 0; v < TEAM; v++)
+            {
+                const int k = team_count[v];
+                if (v < w) start += k;
+                kh += k;
+                most = max(most, k);
+                any_image |= (unsigned)team_image[v];
+            }
+            if (most > kPruneStage)
+            {
+                // a share that does not fit its staging: one warp for all
+                if (w == 0) kh = walk(0, T, wc, usable);
+            }
+            else
+                for (int k = lane; k < kept; k += 32)
+                    if (start + k < usable) wc[start + k] = stage[k];
+            if (w != 0) continue;
         }
         // an overflowed cluster keeps no list (the flag makes the caller regrow
         // and rebuild); otherwise pad it to a whole window
-        if (kh > usable) kh = 0;
+        if (kh > usable)
+        {
+            if (lane == 0) atomicOr(&counters[kCntOverflow], kOvfWords);
+            kh = 0;
+        }
         const int hp = (kh + kWindow - 1) & ~(kWindow - 1);
         const unsigned null_word = (unsigned)s0 - slot0;
         for (int k2 = kh + lane; k2 < hp; k2 += 32) wc[k2] = null_word;
@@ -975,9 +1025,13 @@ int launch_pack(const ForceInputs& in, cudaStream_t s, const int* gate)
 int launch_prune(const ForceInputs& in, cudaStream_t s)
 {
     spgnb_nl* nl = in.nl;
-    const int prune_bps = in.prune_blocks_per_sm > 0 ? in.prune_blocks_per_sm : 5;
-    const int grid = std::max(1, std::min(num_sms() * prune_bps, (nl->clusters_cap + kPruneWarps - 1) / kPruneWarps));
-    launch_dependent(k_prune8, grid, kPruneWarps * 32, 0, s, in.p0, in.d_fps, nl->opt.prune_buffer, nl->d_counters,
+    // the blocks-per-SM setting counts blocks of eight warps
+    const int prune_bps = 2 * (in.prune_blocks_per_sm > 0 ? in.prune_blocks_per_sm : 5);
+    // a block of four warps per cluster while there is room for that many
+    const bool team = nl->clusters_cap <= num_sms() * 16;
+    const int grid = std::max(1, std::min(num_sms() * prune_bps, team ? nl->clusters_cap :
+                                                                 (nl->clusters_cap + kPruneWarps - 1) / kPruneWarps));
+    launch_dependent(team ? k_prune8<4> : k_prune8<1>, grid, kPruneWarps * 32, 0, s, in.p0, in.d_fps, nl->opt.prune_buffer, nl->d_counters,
                                                nl->clusters_cap, nl->table_cap, nl->list_cap,
                                                nl->d_cl_sys, nl->d_sys, nl->d_tcount, nl->d_tab, nl->d_tmask,
                                                in.slot_pos, nl->d_pref, nl->d_pcount, nl->d_pwords, nl->S,
