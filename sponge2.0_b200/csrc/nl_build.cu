@@ -71,6 +71,7 @@ __global__ void k_check_refresh(int n_slots, const int* __restrict__ slot_atom, 
                                 const SysDesc* __restrict__ sys, const float3* __restrict__ crd,
                                 const float4* __restrict__ x0, int* __restrict__ need, int* counters)
 {
+    grid_dep_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     bool move = false;
     if (s < n_slots)
@@ -103,6 +104,7 @@ __global__ void k_bin(int n, const float3* __restrict__ crd, const int* __restri
                       float4* __restrict__ wrapped, int* __restrict__ cell_count, const int* __restrict__ need,
                       const int* __restrict__ counters)
 {
+    grid_dep_wait();
     if (counters[kCntNeed] == 0) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || !need[atom_sys[i]]) return;
@@ -136,6 +138,7 @@ __global__ void k_scan_cells(const SysDesc* __restrict__ sys, const int* __restr
                              int2* __restrict__ cell_cl, int max_atom_in_grid, const int* __restrict__ need,
                              int* __restrict__ ncl, int* counters)
 {
+    grid_dep_wait();
     const int sy = blockIdx.x;
     if (counters[kCntNeed] == 0 || !need[sy]) return;
     const SysDesc& g = sys[sy];
@@ -171,6 +174,7 @@ __global__ void k_scatter(int n, const int* __restrict__ atom_sys, const int* __
                           const SysDesc* __restrict__ sys, int* __restrict__ cell_cursor, int* __restrict__ tmp_atoms,
                           const int* __restrict__ need, const int* __restrict__ counters)
 {
+    grid_dep_wait();
     if (counters[kCntNeed] == 0) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -196,6 +200,7 @@ __global__ void k_sort_cells(int G, const int* __restrict__ cell_sys, const SysD
                              const float4* __restrict__ wrapped, int* __restrict__ slot_atom, int* __restrict__ cl_cell,
                              int* __restrict__ atom_slot, const int* __restrict__ need, const int* __restrict__ counters)
 {
+    grid_dep_wait();
     if (counters[kCntNeed] == 0) return;
     extern __shared__ unsigned long long keys[];
     for (int c = blockIdx.x; c < G; c += gridDim.x)
@@ -257,6 +262,7 @@ __global__ void k_cluster_props(const float3* __restrict__ crd, int* __restrict_
                                 const int* __restrict__ need, const int* __restrict__ ncl, int* __restrict__ tcount,
                                 int* __restrict__ pcount)
 {
+    grid_dep_wait();
     if (counters[kCntNeed] == 0) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int k = t >> 3;
@@ -468,6 +474,7 @@ __device__ __forceinline__ int ex_reach(int g, int2 e)
 template <int TEAM>
 __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlocks) k_search(const SearchArgs A)
 {
+    grid_dep_wait();
     if (A.go && *A.go == 0) return;
     __shared__ SearchOwn own_all[kSearchWarps];
     __shared__ int queue_all[kSearchWarps][kSearchQueue];  // surviving candidates {cluster | stencil flags << 28}
@@ -837,6 +844,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlock
 // rebuild.
 __global__ void k_rev_clear(int clusters_cap, int* __restrict__ rev_count, const int* __restrict__ need)
 {
+    grid_dep_wait();
     if (need && *need == 0) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < clusters_cap) rev_count[c] = 0;
@@ -846,6 +854,7 @@ __global__ void k_rev_fill(int clusters_cap, int table_cap, const int* __restric
                            const float4* __restrict__ tab, int* __restrict__ rev, int* __restrict__ rev_count,
                            int* counters, const int* __restrict__ need)
 {
+    grid_dep_wait();
     if (need && *need == 0) return;
     const int lane = threadIdx.x & 31;
     const int warps = gridDim.x * (blockDim.x >> 5);
@@ -872,6 +881,7 @@ constexpr int kRevWarps = 4;
 __global__ void k_rev_sort(int clusters_cap, int table_cap, int* __restrict__ rev, const int* __restrict__ rev_count,
                            const int* __restrict__ need)
 {
+    grid_dep_wait();
     if (need && *need == 0) return;
     extern __shared__ int rev_buf[];  // kRevWarps x table_cap
     const int lane = threadIdx.x & 31;
@@ -898,6 +908,7 @@ __global__ void k_rev_sort(int clusters_cap, int table_cap, int* __restrict__ re
 // its owner (the lower atom_local index) as the reference stores it.
 __global__ void k_export_zero(int n, spgnb_atom_group* __restrict__ nl, const int* __restrict__ counters)
 {
+    grid_dep_wait();
     if (counters[kCntNeed] == 0) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n)
@@ -933,6 +944,7 @@ __global__ void k_export_lists(int clusters_cap, int table_cap, const int* __res
                                int ovf_bits, const int* __restrict__ need, const int* __restrict__ rev,
                                const int* __restrict__ rev_count)
 {
+    grid_dep_wait();
     if (HALF && *need == 0) return;
     // an atom's kept partners of a chunk, compacted here so that its list is
     // written with contiguous stores (blocks of 128 threads)
@@ -1076,6 +1088,7 @@ __global__ void k_export_lists(int clusters_cap, int table_cap, const int* __res
 
 __global__ void k_zero_groups(int n, spgnb_atom_group* __restrict__ g)
 {
+    grid_dep_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n)
     {
@@ -1088,6 +1101,7 @@ __global__ void k_finish(int G, int S, const int* __restrict__ cell_sys, const i
                          int* __restrict__ prune, int* __restrict__ cell_count, int* __restrict__ cell_cursor,
                          int* counters)
 {
+    grid_dep_wait();
     if (counters[kCntNeed] == 0) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < G && need[cell_sys[c]])
@@ -1103,38 +1117,49 @@ __global__ void k_finish(int G, int S, const int* __restrict__ cell_sys, const i
     }
 }
 
-// Refresh by a fixed interval of steps (NEIGHBOR_LIST::Update with
-// refresh_interval > 0), counted on the device per system: a system rebuilds
-// when its own step count reaches a multiple of the interval, so a system's
-// rebuilds do not depend on when it joined a batch.
-__global__ void k_interval_need(int S, int interval, const int* __restrict__ steps, const int* __restrict__ live,
-                                const int* __restrict__ active, int* __restrict__ need, int* counters)
+__device__ __forceinline__ void reset_list_counters(int* counters)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const bool due = interval > 0 && live[s] && (!active || active[s] != 0) && (steps[s] + 1) % interval == 0;
-    need[s] = due ? 1 : 0;
-    if (due) counters[kCntNeed] = 1;
+    counters[kCntItems] = 0;
+    counters[kCntEntries] = 0;
+    counters[kCntEntries + 1] = 0;
+    counters[kCntWords] = 0;
+    counters[kCntWords + 1] = 0;
+    counters[kCntPWordsLast] = 0;
+    counters[kCntPWordsLast + 1] = 0;
+    counters[kCntSearchNext] = 0;
 }
 
-__global__ void k_set_need(int S, const int* __restrict__ live, const int* __restrict__ active,
-                           int* __restrict__ need, int* counters)
+__global__ void k_reset_list_counters(int* counters)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const bool due = live[s] && (!active || active[s] != 0);
-    need[s] = due ? 1 : 0;
-    if (due) counters[kCntNeed] = 1;
+    grid_dep_wait();
+    if (counters[kCntNeed] != 0) reset_list_counters(counters);
 }
 
-__global__ void k_need_preset(int S, const int* __restrict__ flags, const int* __restrict__ live,
-                              int* __restrict__ need, int* counters)
+// The rebuild decision that needs no look at the atoms, for every system, and
+// the list counters' reset when some system rebuilds; one block.
+//   kBuildForced: every live system.
+//   kBuildInterval: refresh by a fixed interval of steps (NEIGHBOR_LIST::Update
+//   with refresh_interval > 0), counted on the device per system: a system
+//   rebuilds when its own step count (aux) reaches a multiple of the interval,
+//   so its rebuilds do not depend on when it joined a batch.
+//   kBuildPreset: the systems flagged in aux.
+__global__ void k_decide(int how, int S, int interval, const int* __restrict__ aux, const int* __restrict__ live,
+                         const int* __restrict__ active, int* __restrict__ need, int* counters)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const bool due = live[s] && flags[s];
-    need[s] = due ? 1 : 0;
-    if (due) counters[kCntNeed] = 1;
+    grid_dep_wait();
+    int any = 0;
+    for (int s = threadIdx.x; s < S; s += blockDim.x)
+    {
+        bool due = live[s] && (how == kBuildPreset || !active || active[s] != 0);
+        if (how == kBuildInterval) due = due && interval > 0 && (aux[s] + 1) % interval == 0;
+        if (how == kBuildPreset) due = due && aux[s];
+        need[s] = due ? 1 : 0;
+        any |= due ? 1 : 0;
+    }
+    any = __syncthreads_or(any);
+    if (threadIdx.x != 0) return;
+    counters[kCntNeed] = any;
+    if (any) reset_list_counters(counters);
 }
 
 __global__ void k_prune_live(int S, const int* __restrict__ live, int* __restrict__ prune, int* counters)
@@ -1155,23 +1180,11 @@ __global__ void k_fill_int(int* __restrict__ p, long long n, int v)
 // cluster counter and the table statistics start again.
 __global__ void k_sym_begin(int* counters)
 {
+    grid_dep_wait();
     counters[kCntEntries] = 0;
     counters[kCntEntries + 1] = 0;
     counters[kCntWords] = 0;
     counters[kCntWords + 1] = 0;
-    counters[kCntSearchNext] = 0;
-}
-
-__global__ void k_reset_list_counters(int* counters)
-{
-    if (counters[kCntNeed] == 0) return;
-    counters[kCntItems] = 0;
-    counters[kCntEntries] = 0;
-    counters[kCntEntries + 1] = 0;
-    counters[kCntWords] = 0;
-    counters[kCntWords + 1] = 0;
-    counters[kCntPWordsLast] = 0;
-    counters[kCntPWordsLast + 1] = 0;
     counters[kCntSearchNext] = 0;
 }
 
@@ -1227,9 +1240,9 @@ int launch_search(const spgnb_nl* nl, const int* need, const int* ex_start, cons
     a.two_sided_atoms = two_sided;
     const int ccap = nl->clusters_cap, sms = num_sms();
     if (ccap <= sms * 16)
-        k_search<4><<<std::max(1, std::min(ccap, sms * 8)), kSearchWarps * 32, 0, s>>>(a);
+        launch_dependent(k_search<4>, std::max(1, std::min(ccap, sms * 8)), kSearchWarps * 32, 0, s, a);
     else
-        k_search<1><<<std::max(1, std::min((ccap + kSearchWarps - 1) / kSearchWarps, sms * 8)), kSearchWarps * 32, 0, s>>>(a);
+        launch_dependent(k_search<1>, std::max(1, std::min((ccap + kSearchWarps - 1) / kSearchWarps, sms * 8)), kSearchWarps * 32, 0, s, a);
     SPGNB_CHECK_LAUNCH("k_search");
     return SPGNB_OK;
 }
@@ -1416,14 +1429,14 @@ int build_rev(const spgnb_nl* nl, cudaStream_t s, const int* need)
         return fail(SPGNB_E_UNSUPPORTED, "neighbour list: %d table elements per cluster exceed the reverse index's "
                                          "sort", nl->table_cap);
     const int warp_blocks = std::max(1, std::min((ccap + kRevWarps - 1) / kRevWarps, num_sms() * 16));
-    k_rev_clear<<<(ccap + 255) / 256, 256, 0, s>>>(ccap, nl->d_rev_count, need);
+    launch_dependent(k_rev_clear, (ccap + 255) / 256, 256, 0, s, ccap, nl->d_rev_count, need);
     SPGNB_CHECK_LAUNCH("k_rev_clear");
-    k_rev_fill<<<warp_blocks, kRevWarps * 32, 0, s>>>(ccap, nl->table_cap, nl->d_tcount, nl->d_tab, nl->d_rev,
+    launch_dependent(k_rev_fill, warp_blocks, kRevWarps * 32, 0, s, ccap, nl->table_cap, nl->d_tcount, nl->d_tab, nl->d_rev,
                                                       nl->d_rev_count, nl->d_counters, need);
     SPGNB_CHECK_LAUNCH("k_rev_fill");
     if (smem > 48 * 1024)
         SPGNB_CUDA(cudaFuncSetAttribute(k_rev_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_rev_sort<<<warp_blocks, kRevWarps * 32, smem, s>>>(ccap, nl->table_cap, nl->d_rev, nl->d_rev_count, need);
+    launch_dependent(k_rev_sort, warp_blocks, kRevWarps * 32, smem, s, ccap, nl->table_cap, nl->d_rev, nl->d_rev_count, need);
     SPGNB_CHECK_LAUNCH("k_rev_sort");
     nl->rev_built = true;
     return SPGNB_OK;
@@ -1882,6 +1895,9 @@ int nl_create_multi(int n_systems, const int* atom_counts, const spgnb_ltmatrix3
     return SPGNB_OK;
 }
 
+int queue_clusters(spgnb_nl* nl, int n, const float3* d_crd, const int* d_atom_local, const int* ex_start,
+                   const int* ex_list, const int* ex_num, cudaStream_t s);
+
 // Queues one rebuild, or the device-side decision about one, on stream s.
 // how: kBuildForced rebuilds every live system, kBuildSkin lets each
 // system's skin check decide, kBuildInterval rebuilds a system when its step
@@ -1892,55 +1908,51 @@ int nl_queue_build(spgnb_nl* nl, int n, const float3* d_crd, const int* d_atom_l
                    const int* d_active)
 {
     const int slots_cap = nl->clusters_cap * kClusterSize;
-    const int sb = (nl->S + 255) / 256;
     if (how != kBuildSkin)
     {
         if ((how == kBuildInterval || how == kBuildPreset) && !d_aux)
             return fail(SPGNB_E_ARG, "nl_queue_build: per-system steps or flags missing");
-        SPGNB_CUDA(cudaMemsetAsync(nl->d_counters + kCntNeed, 0, sizeof(int), s));
-        if (how == kBuildForced)
-            k_set_need<<<sb, 256, 0, s>>>(nl->S, nl->d_live, d_active, nl->d_need, nl->d_counters);
-        else if (how == kBuildInterval)
-            k_interval_need<<<sb, 256, 0, s>>>(nl->S, interval, d_aux, nl->d_live, d_active, nl->d_need,
-                                               nl->d_counters);
-        else
-            k_need_preset<<<sb, 256, 0, s>>>(nl->S, d_aux, nl->d_live, nl->d_need, nl->d_counters);
-        SPGNB_CHECK_LAUNCH("k_need");
+        launch_dependent(k_decide, 1, 256, 0, s, how, nl->S, interval, d_aux, nl->d_live, d_active, nl->d_need,
+                         nl->d_counters);
+        SPGNB_CHECK_LAUNCH("k_decide");
+        return queue_clusters(nl, n, d_crd, d_atom_local, ex_start, ex_list, ex_num, s);
     }
-    else
-    {
-        SPGNB_CUDA(cudaMemsetAsync(nl->d_counters + kCntNeed, 0, sizeof(int), s));
-        SPGNB_CUDA(cudaMemsetAsync(nl->d_need, 0, sizeof(int) * nl->S, s));
-        k_check_refresh<<<(slots_cap + 255) / 256, 256, 0, s>>>(slots_cap, nl->d_slot_atom, nl->d_cl_sys, nl->d_sys,
-                                                                  d_crd, nl->d_slot_x0, nl->d_need, nl->d_counters);
-        SPGNB_CHECK_LAUNCH("k_check_refresh");
-    }
+    SPGNB_CUDA(cudaMemsetAsync(nl->d_counters + kCntNeed, 0, sizeof(int), s));
+    SPGNB_CUDA(cudaMemsetAsync(nl->d_need, 0, sizeof(int) * nl->S, s));
+    launch_dependent(k_check_refresh, (slots_cap + 255) / 256, 256, 0, s, slots_cap, nl->d_slot_atom, nl->d_cl_sys,
+                     nl->d_sys, d_crd, nl->d_slot_x0, nl->d_need, nl->d_counters);
+    SPGNB_CHECK_LAUNCH("k_check_refresh");
     return nl_queue_build_body(nl, n, d_crd, d_atom_local, ex_start, ex_list, ex_num, s);
 }
 
 int nl_queue_build_body(spgnb_nl* nl, int n, const float3* d_crd, const int* d_atom_local, const int* ex_start,
                         const int* ex_list, const int* ex_num, cudaStream_t s)
 {
+    launch_dependent(k_reset_list_counters, 1, 1, 0, s, nl->d_counters);
+    SPGNB_CHECK_LAUNCH("k_reset_list_counters");
+    return queue_clusters(nl, n, d_crd, d_atom_local, ex_start, ex_list, ex_num, s);
+}
+
+// The build from the binning on, the list counters already reset.
+int queue_clusters(spgnb_nl* nl, int n, const float3* d_crd, const int* d_atom_local, const int* ex_start,
+                   const int* ex_list, const int* ex_num, cudaStream_t s)
+{
     const int sms = num_sms();
     const int slots_cap = nl->clusters_cap * kClusterSize;
     const int ccap = nl->clusters_cap;
-    k_reset_list_counters<<<1, 1, 0, s>>>(nl->d_counters);
-    SPGNB_CHECK_LAUNCH("k_reset_list_counters");
-    k_bin<<<(n + 255) / 256, 256, 0, s>>>(n, d_crd, nl->d_atom_sys, nl->d_sys, nl->d_atom_cell, nl->d_atom_shift,
+    launch_dependent(k_bin, (n + 255) / 256, 256, 0, s, n, d_crd, nl->d_atom_sys, nl->d_sys, nl->d_atom_cell, nl->d_atom_shift,
                                             nl->d_wrapped, nl->d_cell_count, nl->d_need, nl->d_counters);
     SPGNB_CHECK_LAUNCH("k_bin");
-    k_scan_cells<<<nl->S, 1024, 0, s>>>(nl->d_sys, nl->d_cell_count, nl->d_cell_cl, nl->opt.max_atom_in_grid_numbers,
+    launch_dependent(k_scan_cells, nl->S, 1024, 0, s, nl->d_sys, nl->d_cell_count, nl->d_cell_cl, nl->opt.max_atom_in_grid_numbers,
                                          nl->d_need, nl->d_ncl, nl->d_counters);
     SPGNB_CHECK_LAUNCH("k_scan_cells");
-    k_scatter<<<(n + 255) / 256, 256, 0, s>>>(n, nl->d_atom_sys, nl->d_atom_cell, nl->d_cell_cl, nl->d_ncl, nl->d_sys,
+    launch_dependent(k_scatter, (n + 255) / 256, 256, 0, s, n, nl->d_atom_sys, nl->d_atom_cell, nl->d_cell_cl, nl->d_ncl, nl->d_sys,
                                                 nl->d_cell_cursor, nl->d_tmp_atoms, nl->d_need, nl->d_counters);
     SPGNB_CHECK_LAUNCH("k_scatter");
-    k_sort_cells<<<std::min(nl->G, sms * 16), 128, kMaxCellAtoms * sizeof(unsigned long long), s>>>(
-        nl->G, nl->d_cell_sys, nl->d_sys, nl->d_cell_count, nl->d_cell_cl, nl->d_ncl, nl->d_tmp_atoms, nl->d_wrapped,
+    launch_dependent(k_sort_cells, std::min(nl->G, sms * 16), 128, kMaxCellAtoms * sizeof(unsigned long long), s, nl->G, nl->d_cell_sys, nl->d_sys, nl->d_cell_count, nl->d_cell_cl, nl->d_ncl, nl->d_tmp_atoms, nl->d_wrapped,
         nl->d_slot_atom, nl->d_cl_cell, nl->d_atom_slot, nl->d_need, nl->d_counters);
     SPGNB_CHECK_LAUNCH("k_sort_cells");
-    k_cluster_props<<<(slots_cap + 255) / 256, 256, 0, s>>>(
-        d_crd, nl->d_slot_atom, nl->d_atom_shift, d_atom_local, nl->d_cl_sys, nl->d_sys, nl->d_counters, nl->d_cl_u,
+    launch_dependent(k_cluster_props, (slots_cap + 255) / 256, 256, 0, s, d_crd, nl->d_slot_atom, nl->d_atom_shift, d_atom_local, nl->d_cl_sys, nl->d_sys, nl->d_counters, nl->d_cl_u,
         nl->d_cl_q, nl->d_cl_c, nl->d_slot_x0, nl->d_slot_gid, nl->d_slot_d0, nl->d_slot_ex, ex_start, ex_list, ex_num,
         ccap, nl->d_need, nl->d_ncl, nl->d_tcount, nl->d_pcount);
     SPGNB_CHECK_LAUNCH("k_cluster_props");
@@ -1957,17 +1969,16 @@ int nl_queue_build_body(spgnb_nl* nl, int n, const float3* d_crd, const int* d_a
     {
         int st = build_rev(nl, s, nl->d_counters + kCntNeed);
         if (st) return st;
-        k_export_zero<<<(n + 255) / 256, 256, 0, s>>>(n, nl->d_nl, nl->d_counters);
+        launch_dependent(k_export_zero, (n + 255) / 256, 256, 0, s, n, nl->d_nl, nl->d_counters);
         SPGNB_CHECK_LAUNCH("k_export_zero");
-        k_export_lists<true><<<std::max(1, std::min((ccap + 3) / 4, sms * 16)), 128, 0, s>>>(
-            ccap, nl->table_cap, nl->d_tcount, nl->d_tab, nl->d_tmask, nl->d_slot_atom, nl->d_slot_x0, nl->d_slot_gid,
+        launch_dependent(k_export_lists<true>, std::max(1, std::min((ccap + 3) / 4, sms * 16)), 128, 0, s, ccap, nl->table_cap, nl->d_tcount, nl->d_tab, nl->d_tmask, nl->d_slot_atom, nl->d_slot_x0, nl->d_slot_gid,
             nullptr,
             Cell{}, Cell{}, -1.0f, nl->d_nl, nl->opt.max_neighbor_numbers, nl->d_counters + kCntOverflow, kOvfList,
             nl->d_counters + kCntNeed, nl->d_rev, nl->d_rev_count);
         SPGNB_CHECK_LAUNCH("k_export_lists");
     }
     const int fin = std::max(nl->G, nl->S);
-    k_finish<<<(fin + 255) / 256, 256, 0, s>>>(nl->G, nl->S, nl->d_cell_sys, nl->d_need, nl->d_prune,
+    launch_dependent(k_finish, (fin + 255) / 256, 256, 0, s, nl->G, nl->S, nl->d_cell_sys, nl->d_need, nl->d_prune,
                                                   nl->d_cell_count, nl->d_cell_cursor, nl->d_counters);
     SPGNB_CHECK_LAUNCH("k_finish");
     nl->built = true;
@@ -2219,7 +2230,7 @@ namespace spgnb
 // the flagged atoms' clusters.
 int research_last_build(const spgnb_nl* nl, cudaStream_t s, int half, const unsigned char* flags)
 {
-    k_sym_begin<<<1, 1, 0, s>>>(nl->d_counters);
+    launch_dependent(k_sym_begin, 1, 1, 0, s, nl->d_counters);
     SPGNB_CHECK_LAUNCH("k_sym_begin");
     // every live system, whatever the last build flagged: a system's tables
     // are those of its own last build either way
@@ -2273,11 +2284,10 @@ int spgnb_nl_build_full(spgnb_nl* nl, int local_atom_numbers, const spgnb_vector
     if (!nl->rev_built && (st = build_rev(nl, s, nullptr))) return st;
     const int n = local_atom_numbers;
     // atoms in no cluster with a table (none, normally) keep a zero count
-    k_zero_groups<<<(n + 255) / 256, 256, 0, s>>>(n, d_full_nl);
+    launch_dependent(k_zero_groups, (n + 255) / 256, 256, 0, s, n, d_full_nl);
     SPGNB_CHECK_LAUNCH("k_zero_groups");
     const int ccap = nl->clusters_cap;
-    k_export_lists<false><<<std::max(1, std::min((ccap + 3) / 4, num_sms() * 16)), 128, 0, s>>>(
-        ccap, nl->table_cap, nl->d_tcount, nl->d_tab, nl->d_tmask, nl->d_slot_atom, nl->d_slot_x0, nl->d_slot_gid,
+    launch_dependent(k_export_lists<false>, std::max(1, std::min((ccap + 3) / 4, num_sms() * 16)), 128, 0, s, ccap, nl->table_cap, nl->d_tcount, nl->d_tab, nl->d_tmask, nl->d_slot_atom, nl->d_slot_x0, nl->d_slot_gid,
         (const float3*)d_crd, make_cell(cell), make_cell(rcell), cutoff > 0.0f ? cutoff * cutoff : -1.0f, d_full_nl,
         max_neighbor_numbers, d_overflow, 1, nullptr, nl->d_rev, nl->d_rev_count);
     SPGNB_CHECK_LAUNCH("k_export_lists");
