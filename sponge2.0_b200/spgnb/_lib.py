@@ -9,6 +9,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+import numpy as np
+
 PKG_DIR = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 LIB_PATH = os.path.join(PKG_DIR, "libspgnb.so")
 
@@ -57,6 +59,10 @@ class LTMatrix3(C.Structure):
 
     @classmethod
     def of(cls, m):
+        # a step converts the cell six times: a float32 array, which systems
+        # hold it as, is copied as it is (0.3 us; element by element 1.6)
+        if type(m) is np.ndarray and m.dtype == np.float32 and m.shape == (6,) and m.flags.c_contiguous:
+            return cls.from_buffer_copy(m)
         m = [float(v) for v in m]
         return cls(*m)
 

@@ -33,7 +33,9 @@ def _ptr(t):
 
 
 def _bind_stream():
-    lib().spgnb_set_stream(C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    # the current stream's handle without a Stream object around it (three
+    # times a step)
+    lib().spgnb_set_stream(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _controller_int(controller, key, default):
@@ -327,15 +329,17 @@ class SOLVENT_LENNARD_JONES:
                                                          atom_direct_pme_energy):
         if not self.is_initialized:
             return
+        arrays = [_ptr(t) for t in (d_res_start, crd, charge, frc, atom_energy, atom_lj_virial,
+                                    atom_direct_pme_energy)]
+        cells = LTMatrix3.of(cell), LTMatrix3.of(rcell)
+        if isinstance(nl, NEIGHBOR_LIST) and nl.handle is not None:
+            return  # over an spgnb list the LJ module's call evaluates the waters too
         _bind_stream()
-        spg = nl.handle if isinstance(nl, NEIGHBOR_LIST) else None
-        groups = None if spg is not None else int(nl)
         check(lib().spgnb_solvent_pme_direct_force(self.handle, int(atom_numbers), int(residue_numbers),
-                                                   _ptr(d_res_start), _ptr(crd), _ptr(charge), _ptr(frc),
-                                                   LTMatrix3.of(cell), LTMatrix3.of(rcell), spg, groups,
-                                                   float(pme_beta), int(need_atom_energy), _ptr(atom_energy),
-                                                   int(need_virial), _ptr(atom_lj_virial),
-                                                   _ptr(atom_direct_pme_energy)))
+                                                   *arrays[:4], *cells, None,
+                                                   None if isinstance(nl, NEIGHBOR_LIST) else int(nl),
+                                                   float(pme_beta), int(need_atom_energy), arrays[4],
+                                                   int(need_virial), arrays[5], arrays[6]))
 
     def Clear(self):
         if self.handle is not None:
