@@ -80,8 +80,7 @@ struct spgnb_batch
     int* d_left = nullptr;            // per system: steps left (-1 unlimited, 0 stopped or parked)
     int* d_flags = nullptr;           // per system: evaluate now
     std::vector<int> h_flags;
-    float4* d_slot_pos = nullptr;
-    int4* d_slot_aux = nullptr;
+    spgnb::SlotRec* d_slots = nullptr;
     // stepping
     bool have_water = false;
     float ra = 0, rb = 0, rc = 0, mO = 0, mH = 0;
@@ -199,7 +198,7 @@ struct StepArgs
     const spgnb::SysDesc* sys;
     const float4* slot_x0;
     const float4* slot_d0;
-    float4* slot_pos;
+    spgnb::SlotRec* slots;
     const float4* pref;             // positions at the last pruning (null: pruning off)
     float half_buffer2;
     int* prune;
@@ -298,7 +297,7 @@ __device__ __forceinline__ void pack_atom(const StepArgs& a, const AtomIn& t, in
         dy -= sy2 * D.cell.a22 + sz * D.cell.a32;
         dz -= sz * D.cell.a33;
         const float4 p = make_float4(t.d0.x + dx, t.d0.y + dy, t.d0.z + dz, t.q);
-        a.slot_pos[t.slot] = p;
+        a.slots[t.slot].pos = p;
         if (a.pref)
         {
             const float ex = p.x - t.pref.x, ey = p.y - t.pref.y, ez = p.z - t.pref.z;
@@ -513,8 +512,7 @@ ForceInputs batch_inputs(spgnb_batch* b, int mode, const int* only)
     in.crd = b->d_crd;
     in.charge = b->d_charge;
     in.atom_type = b->d_type;
-    in.slot_pos = b->d_slot_pos;
-    in.slot_aux = b->d_slot_aux;
+    in.slots = b->d_slots;
     in.p0 = b->h_fps[0];
     in.d_fps = b->d_fps;
     in.fit = b->fit;
@@ -642,7 +640,7 @@ int batch_step(spgnb_batch* b, bool energy, cudaStream_t s, CaptureIf* cap = nul
     a.sys = nl->d_sys;
     a.slot_x0 = nl->d_slot_x0;
     a.slot_d0 = nl->d_slot_d0;
-    a.slot_pos = b->d_slot_pos;
+    a.slots = b->d_slots;
     const bool track = nl->opt.prune_buffer > 0.0f;
     a.pref = track ? nl->d_pref : nullptr;
     const float half = 0.5f * nl->opt.prune_buffer;
@@ -794,8 +792,7 @@ void free_batch(spgnb_batch* b)
     dfree(b->d_steps);
     dfree(b->d_left);
     dfree(b->d_flags);
-    dfree(b->d_slot_pos);
-    dfree(b->d_slot_aux);
+    dfree(b->d_slots);
     dfree(b->d_t4);
     if (b->stream) cudaStreamSynchronize(b->stream);
     for (PinnedStage& ps : b->stages)
@@ -1021,8 +1018,7 @@ int create_common(spgnb_batch* b, const NLPoolSpec& spec, long long ex_cap, int 
         (st = zalloc(&b->d_in_water, n)) || (st = dalloc(&b->d_lambda, S1)) || (st = zalloc(&b->d_skin_hit, S1)) ||
         (st = zalloc(&b->d_done, 1)) ||
         (st = zalloc(&b->d_steps, S1)) || (st = zalloc(&b->d_left, S1)) || (st = zalloc(&b->d_flags, S1)) ||
-        (st = dalloc(&b->d_slot_pos, (size_t)b->nl->clusters_cap * kClusterSize + 1)) ||
-        (st = dalloc(&b->d_slot_aux, (size_t)b->nl->clusters_cap * kClusterSize + 1)))
+        (st = dalloc(&b->d_slots, (size_t)b->nl->clusters_cap * kClusterSize + 1)))
         return st;
     SPGNB_CUDA(cudaMemcpy(b->d_t4, t4.data(), sizeof(float4) * t4.size(), cudaMemcpyHostToDevice));
     SPGNB_CUDA(cudaMemset(b->d_waters, 0xff, sizeof(int) * b->w_cap));

@@ -57,7 +57,7 @@ __global__ void k_pack_slots(int slots_cap, int* counters, const int* __restrict
                              const SysDesc* __restrict__ sys, const int4* __restrict__ cl_q,
                              const float4* __restrict__ x0, const float4* __restrict__ d0,
                              const float3* __restrict__ crd, const float* __restrict__ charge,
-                             const int* __restrict__ local_type, float4* __restrict__ pos, int4* __restrict__ aux,
+                             const int* __restrict__ local_type, SlotRec* __restrict__ rec,
                              const float4* __restrict__ pref, float half_buffer2, int* __restrict__ prune,
                              long long* __restrict__ clear_totals, long long* __restrict__ clear_one,
                              float* __restrict__ clear_a, float* __restrict__ clear_b, int clear_n,
@@ -77,8 +77,8 @@ __global__ void k_pack_slots(int slots_cap, int* counters, const int* __restrict
     }
     if (s == slots_cap)
     {
-        pos[s] = make_float4(1.0e4f, 1.0e4f, 1.0e4f, 0.0f);
-        aux[s] = make_int4(0, 0, 0, -1);
+        rec[s].pos = make_float4(1.0e4f, 1.0e4f, 1.0e4f, 0.0f);
+        rec[s].aux = make_int4(0, 0, 0, -1);
     }
     else if (s < slots_cap)
     {
@@ -109,8 +109,8 @@ __global__ void k_pack_slots(int slots_cap, int* counters, const int* __restrict
                 if (moved) prune[cl_sys[s >> 3]] = 1;
             }
         }
-        pos[s] = p;
-        aux[s] = make_int4((q.x & 0x3fffff) | (t << 22), q.y, q.z, a >= 0 ? slot_gid[s] : -1);
+        rec[s].pos = p;
+        rec[s].aux = make_int4((q.x & 0x3fffff) | (t << 22), q.y, q.z, a >= 0 ? slot_gid[s] : -1);
     }
     if (__any_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) counters[kCntPrune] = 1;
 }
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
     k_prune8(ForceParams p0, const ForceParams* __restrict__ fps, float buffer, int* counters, int clusters_cap,
              int table_cap, int list_cap, const int* __restrict__ cl_sys, const SysDesc* __restrict__ sys,
              const int* __restrict__ tcount, const float4* __restrict__ tab, const uint2* __restrict__ tmask,
-             const float4* __restrict__ pos, float4* __restrict__ pref, int* __restrict__ lcount,
+             const SlotRec* __restrict__ rec, float4* __restrict__ pref, int* __restrict__ lcount,
              unsigned* __restrict__ words, int n_sys, int* __restrict__ prune)
 {
     grid_dep_wait();
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
         __syncwarp();
         if (lane < kClusterSize)
         {
-            const float4 pl = pos[s0 + lane];
+            const float4 pl = rec[s0 + lane].pos;
             own[0][lane] = -pl.x;
             own[1][lane] = -pl.y;
             own[2][lane] = -pl.z;
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
                     float4 pjs[kPruneAhead];
 #pragma unroll
                     for (int k = 0; k < kPruneAhead; k++)
-                        pjs[k] = pos[(__float_as_int(ent[4 * (g + k) + e_lane].w) & 0x3fffffff) + b_lane];
+                        pjs[k] = rec[(__float_as_int(ent[4 * (g + k) + e_lane].w) & 0x3fffffff) + b_lane].pos;
 #pragma unroll
                     for (int k = 0; k < kPruneAhead; k++)
                     {
@@ -417,10 +417,10 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
 // finishing pass turns the staging into the per-atom arrays and totals.
 template <int MODE, int FIT, bool TRI>
 __global__ void __launch_bounds__(32, kPairResident[MODE])
-    k_pair8(ForceParams p0, const ForceParams* __restrict__ fps, const SysDesc* __restrict__ sys, int n_clusters,
+    k_pair8(ForceParams p0, const EwaldPoly ep, const ForceParams* __restrict__ fps, const SysDesc* __restrict__ sys, int n_clusters,
             int shift, int list_cap, const int* __restrict__ cl_sys, const int* __restrict__ lcount,
-            const unsigned* __restrict__ words, const int4* __restrict__ cl_q, const float4* __restrict__ pos,
-            const int4* __restrict__ aux, const float4* __restrict__ t4, long long* __restrict__ facc,
+            const unsigned* __restrict__ words, const int4* __restrict__ cl_q, const SlotRec* __restrict__ rec,
+            const float4* __restrict__ t4, long long* __restrict__ facc,
             long long* __restrict__ oacc, long long* __restrict__ totals, const int* __restrict__ only)
 {
     grid_dep_wait();
@@ -453,8 +453,8 @@ __global__ void __launch_bounds__(32, kPairResident[MODE])
     // rows of its four atom pairs against every partner type,
     // {-A_a, -A_b, B_a, B_b}, staged in shared memory
     {
-        const float4 u = pos[s0 + (lane & 7)];
-        const int4 x = aux[s0 + (lane & 7)];
+        const float4 u = rec[s0 + (lane & 7)].pos;
+        const int4 x = rec[s0 + (lane & 7)].aux;
         if (lane < 8)
         {
             float* f = reinterpret_cast<float*>(&iat[lane >> 1][0]) + (lane & 1);
@@ -496,37 +496,35 @@ __global__ void __launch_bounds__(32, kPairResident[MODE])
         const unsigned* __restrict__ wl = wb + lane;
         unsigned wc = wl[0];
         unsigned wn = iters > 1 ? wl[32] : 0u;
-        float4 pjn = pos[slot0 + (int)(wc & kWordSlotMask)];
-        int4 xjn = aux[slot0 + (int)(wc & kWordSlotMask)];
+        float4 pjn;
+        int4 xjn;
+        load_rec(rec + (slot0 + (int)(wc & kWordSlotMask)), pjn, xjn);
 #pragma unroll 1
         for (int it = 0; it < iters; it++)
         {
-            const float4 pjc = pjn;
-            const int4 xjc = xjn;
             const int jc = slot0 + (int)(wc & kWordSlotMask);
-            unsigned wnn = 0u;
-            if (it + 1 < iters)
-            {
-                const int jn = slot0 + (int)(wn & kWordSlotMask);
-                pjn = pos[jn];
-                xjn = aux[jn];
-                if (it + 2 < iters) wnn = wl[32 * (it + 2)];
-            }
-
-            const float ux = centre_step(xjc.x, ci.x), uy = centre_step(xjc.y, ci.y), uz = centre_step(xjc.z, ci.z);
+            const float ux = centre_step(xjn.x, ci.x), uy = centre_step(xjn.y, ci.y), uz = centre_step(xjn.z, ci.z);
             // the partner in the frame of the cluster's centre
-            float sx = __fmaf_rn(ux, qc.a11, pjc.x);
-            float sy2 = __fmaf_rn(uy, qc.a22, pjc.y);
-            const float sz = __fmaf_rn(uz, qc.a33, pjc.z);
+            float sx = __fmaf_rn(ux, qc.a11, pjn.x);
+            float sy2 = __fmaf_rn(uy, qc.a22, pjn.y);
+            const float sz = __fmaf_rn(uz, qc.a33, pjn.z);
             if (TRI)
             {
                 sx = __fmaf_rn(uy, qc.a21, sx);
                 sx = __fmaf_rn(uz, qc.a31, sx);
                 sy2 = __fmaf_rn(uz, qc.a32, sy2);
             }
-            const int tj = (xjc.x >> 22) & 0x7f;
-            const int gj = xjc.w;
-            const float2 qj = f2(pjc.w);
+            const int tj = (xjn.x >> 22) & 0x7f;
+            const int gj = xjn.w;
+            const float2 qj = f2(pjn.w);
+            // the record is used up: the next one takes its registers
+            unsigned wnn = 0u;
+            if (it + 1 < iters)
+            {
+                const int jn = slot0 + (int)(wn & kWordSlotMask);
+                load_rec(rec + jn, pjn, xjn);
+                if (it + 2 < iters) wnn = wl[32 * (it + 2)];
+            }
             float2 hx, hy, hz;     // the partner's force, negated
             float2 jo[PA ? 8 : 1];                                  // the partner's owned sums
 #pragma unroll
@@ -562,7 +560,7 @@ __global__ void __launch_bounds__(32, kPairResident[MODE])
                 const float4 ab = rows[p * nt + tj];
                 float2 elj, ec;
                 float2 f = pair_scalar2<EN, FIT>(r2, __fmul2_rn(qj, pq), make_float2(ab.x, ab.y),
-                                                 make_float2(ab.z, ab.w), pp, elj, ec);
+                                                 make_float2(ab.z, ab.w), pp, ep, elj, ec);
                 f = make_float2(inA ? f.x : 0.0f, inB ? f.y : 0.0f);
                 fx[p] = __ffma2_rn(f, dx, fx[p]);
                 fy[p] = __ffma2_rn(f, dy, fy[p]);
@@ -626,7 +624,7 @@ __global__ void __launch_bounds__(32, kPairResident[MODE])
                 // the partner's force: minus the sum over the cluster's atoms
                 // (all zero when the word has no pair inside the cutoff)
                 const float jx = hx.x + hx.y, jy = hy.x + hy.y, jz = hz.x + hz.y;
-                if (jx != 0.0f || jy != 0.0f || jz != 0.0f)
+                if ((__float_as_uint(jx) | __float_as_uint(jy) | __float_as_uint(jz)) & 0x7fffffffu)
                 {
                     long long* fa = facc + 3 * (size_t)jc;
                     red_add(fa + 0, __float2ll_rn(jx * -kTwoPow32));
@@ -927,10 +925,27 @@ __global__ void k_fin8_atoms(int n, int slots, const int* __restrict__ atom_slot
     }
 }
 
+// The K (forces) or M (energies) fit in r^2 for this Ewald parameter.
+EwaldPoly scaled_fit(const ForceParams& f, bool energy)
+{
+    EwaldPoly e;
+    const double b = f.beta, w = b * b / (double)SPGNB_EWALD_W_MAX;
+    double np = energy ? -b : -b * b * b, nq = 1.0;
+    for (int k = 0; k < 6; k++, np *= w, nq *= w)
+    {
+        const float p = (float)((energy ? kEwaldMPHost[k] : kEwaldKPHost[k]) * np);
+        const float q = (float)((energy ? kEwaldMQHost[k] : kEwaldKQHost[k]) * nq);
+        e.p[k] = make_float2(p, p);
+        e.q[k] = make_float2(q, q);
+    }
+    return e;
+}
+
 template <int M, int F, bool T>
 int launch_pair(const ForceInputs& in, cudaStream_t s)
 {
     const spgnb_nl* nl = in.nl;
+    const EwaldPoly ep = F == 2 ? scaled_fit(in.p0, M >= 1) : EwaldPoly{};
     const int mt = in.max_types > 0 ? in.max_types : in.p0.n_types;
     size_t smem = sizeof(float4) * std::max(4 * mt, 2 * kSumRow);
     // the blocks-per-SM setting counts blocks of four warps: it holds the
@@ -953,8 +968,8 @@ int launch_pair(const ForceInputs& in, cudaStream_t s)
         SPGNB_CUDA(cudaFuncSetAttribute(k_pair8<M, F, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)smem));
     launch_dependent(k_pair8<M, F, T>, grid, 32, smem, s,
-        in.p0, in.d_fps, nl->d_sys, nl->clusters_cap, shift, nl->list_cap, nl->d_cl_sys, nl->d_pcount, nl->d_pwords,
-        nl->d_cl_q, in.slot_pos, in.slot_aux, in.t4, nl->d_facc, nl->d_oacc, in.totals, in.only);
+        in.p0, ep, in.d_fps, nl->d_sys, nl->clusters_cap, shift, nl->list_cap, nl->d_cl_sys, nl->d_pcount, nl->d_pwords,
+        nl->d_cl_q, in.slots, in.t4, nl->d_facc, nl->d_oacc, in.totals, in.only);
     SPGNB_CHECK_LAUNCH("k_pair8");
     return SPGNB_OK;
 }
@@ -965,10 +980,13 @@ int launch_pair_t(const ForceInputs& in, bool tri, cudaStream_t s)
     return tri ? launch_pair<M, F, true>(in, s) : launch_pair<M, F, false>(in, s);
 }
 
+// FIT 2, the fits scaled to the call's one system, or 1 for several systems;
+// 0 outside the fits' range.
 template <int M>
 int launch_pair_ft(const ForceInputs& in, bool tri, cudaStream_t s)
 {
-    return in.fit ? launch_pair_t<M, 1>(in, tri, s) : launch_pair_t<M, 0>(in, tri, s);
+    if (!in.fit) return launch_pair_t<M, 0>(in, tri, s);
+    return in.d_fps ? launch_pair_t<M, 1>(in, tri, s) : launch_pair_t<M, 2>(in, tri, s);
 }
 
 }  // namespace
@@ -1014,8 +1032,8 @@ int launch_pack(const ForceInputs& in, cudaStream_t s, const int* gate)
     const float half = 0.5f * nl->opt.prune_buffer;
     launch_dependent(k_pack_slots, (slots + 256) / 256, 256, 0, s, slots, nl->d_counters, nl->d_slot_atom, nl->d_slot_gid,
                                                      nl->d_cl_sys, nl->d_sys, nl->d_cl_q, nl->d_slot_x0,
-                                                     nl->d_slot_d0, in.crd, in.charge, in.atom_type, in.slot_pos,
-                                                     in.slot_aux, track ? nl->d_pref : nullptr, half * half,
+                                                     nl->d_slot_d0, in.crd, in.charge, in.atom_type, in.slots,
+                                                     track ? nl->d_pref : nullptr, half * half,
                                                      nl->d_prune, in.clear.totals, in.clear.one, in.clear.a, in.clear.b,
                                                      in.clear.n, gate);
     SPGNB_CHECK_LAUNCH("k_pack_slots");
@@ -1027,14 +1045,15 @@ int launch_prune(const ForceInputs& in, cudaStream_t s)
     spgnb_nl* nl = in.nl;
     // the blocks-per-SM setting counts blocks of eight warps
     const int prune_bps = 2 * (in.prune_blocks_per_sm > 0 ? in.prune_blocks_per_sm : 5);
-    // a block of four warps per cluster while there is room for that many
-    const bool team = nl->clusters_cap <= num_sms() * 16;
+    // a block of four warps per cluster up to 36 clusters an SM (24,000 atoms:
+    // 24 us a pruning, 27 with a warp each)
+    const bool team = nl->clusters_cap <= num_sms() * 36;
     const int grid = std::max(1, std::min(num_sms() * prune_bps, team ? nl->clusters_cap :
                                                                  (nl->clusters_cap + kPruneWarps - 1) / kPruneWarps));
     launch_dependent(team ? k_prune8<4> : k_prune8<1>, grid, kPruneWarps * 32, 0, s, in.p0, in.d_fps, nl->opt.prune_buffer, nl->d_counters,
                                                nl->clusters_cap, nl->table_cap, nl->list_cap,
                                                nl->d_cl_sys, nl->d_sys, nl->d_tcount, nl->d_tab, nl->d_tmask,
-                                               in.slot_pos, nl->d_pref, nl->d_pcount, nl->d_pwords, nl->S,
+                                               in.slots, nl->d_pref, nl->d_pcount, nl->d_pwords, nl->S,
                                                nl->d_prune);
     SPGNB_CHECK_LAUNCH("k_prune8");
     return SPGNB_OK;

@@ -183,6 +183,15 @@ struct SysDesc
     Cell qcell;     // cell / 2^22: Cartesian length of one step of the 22-bit cluster centres
 };
 
+// A slot's record for the force pass: its offset from the cluster's centre
+// {delta + displacement, q}, and {centre x | LJ type << 22, centre y, centre
+// z, global index}.  One 32-byte sector, so a partner's gather touches one.
+struct __align__(32) SlotRec
+{
+    float4 pos;
+    int4 aux;
+};
+
 // Pair-function parameters of one system.
 struct ForceParams
 {
@@ -386,8 +395,7 @@ struct spgnb_lj
     float4* d_pos = nullptr;         // per slot (spgnb list) or per atom (atom-group path)
     int* d_pos_type = nullptr;
     int pos_cap = 0;
-    float4* d_sdata = nullptr;       // spgnb list: per-step slot offsets and charges (+ the null slot)
-    int4* d_slot_aux = nullptr;      // per slot: {centre x | LJ type << 22, centre y, centre z, global index}
+    spgnb::SlotRec* d_sdata = nullptr;  // spgnb list: per-step slot records (+ the null slot)
     int sdata_cap = 0;
     int local_atoms = 0;
     bool have_energy = false, have_virial = false;
@@ -501,8 +509,7 @@ struct ForceInputs
     const float3* crd = nullptr;       // per atom, the list's atom order
     const float* charge = nullptr;
     const int* atom_type = nullptr;    // into the LJ table
-    float4* slot_pos = nullptr;        // scratch, slots + 1
-    int4* slot_aux = nullptr;          // scratch, slots + 1
+    SlotRec* slots = nullptr;          // scratch, slots + 1
     ForceParams p0{};                  // the one system's parameters (d_fps null)
     const ForceParams* d_fps = nullptr;  // per system (several systems)
     bool fit = true;                   // every system inside the rational fits' range

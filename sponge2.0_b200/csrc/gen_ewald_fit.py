@@ -129,6 +129,7 @@ def main():
     fmt2 = lambda a: ", ".join(f"{{{float(v):.9e}f, {float(v):.9e}f}}" for v in a)
     for name, a in (("KP", kp2), ("KQ", kq2), ("MP", mp2), ("MQ", mq2)):
         print(f"static __constant__ float2 kEwald{name}2[{len(a)}] = {{{fmt2(a)}}};")
+        print(f"static const double kEwald{name}Host[{len(a)}] = {{{', '.join(repr(float(v)) for v in a)}}};")
 
 
 if __name__ == "__main__":

@@ -444,10 +444,8 @@ int ensure_slots(spgnb_lj* lj, int slots)
 {
     if (slots + 1 <= lj->sdata_cap) return SPGNB_OK;
     dfree(lj->d_sdata);
-    dfree(lj->d_slot_aux);
     int st;
     if ((st = dalloc(&lj->d_sdata, (size_t)(slots + 1)))) return st;
-    if ((st = dalloc(&lj->d_slot_aux, (size_t)(slots + 1)))) return st;
     lj->sdata_cap = slots + 1;
     return SPGNB_OK;
 }
@@ -618,8 +616,7 @@ int spgnb_lj_pme_direct_force(spgnb_lj* lj, int atom_numbers, int local_atom_num
     in.crd = (const float3*)d_crd;
     in.charge = d_charge;
     in.atom_type = lj->d_local_type;
-    in.slot_pos = lj->d_sdata;
-    in.slot_aux = lj->d_slot_aux;
+    in.slots = lj->d_sdata;
     in.p0 = make_pair_const(lj, pme_beta);
     in.fit = in.p0.use_fit != 0;
     in.t4 = lj->d_t4;
@@ -897,7 +894,6 @@ int spgnb_lj_destroy(spgnb_lj* lj)
     dfree(lj->d_pos);
     dfree(lj->d_pos_type);
     dfree(lj->d_sdata);
-    dfree(lj->d_slot_aux);
     dfree(lj->d_t4);
     delete lj;
     return SPGNB_OK;

@@ -96,6 +96,12 @@ __device__ __forceinline__ float rcp_approx(float x)
     return y;
 }
 
+// A fit's numerator and denominator as polynomials in r^2, (c, c) pairs.
+struct EwaldPoly
+{
+    float2 p[6], q[6];
+};
+
 // One system's pair-function parameters as (v, v) pairs, made once per atom
 // pair and kept in registers over its list.
 struct PairParams2
@@ -124,35 +130,44 @@ __device__ __forceinline__ PairParams2 pack_params(const ForceParams& pc)
 // beta^3 K(w) = beta (M(w) - 2/sqrt(pi) exp(-w)) / r^2, so
 //   F_c/qq = (t + beta 2/sqrt(pi) exp(-w)) / r^2,  E_c/qq = t,  t = 1/r - beta M(w).
 // e_lj comes out as -12 E_lj and e_c as -E_c; the kernels scale the sums once.
+// FIT 1: the fits in w / W_MAX; FIT 2: the same fits as polynomials in r^2
+// with -beta^3 (K) or -beta (M) in the numerator, ep, made for the one system
+// of a call: two packed instructions fewer a pair.  FIT 0: erfc.
 template <bool ENERGY, int FIT>
 __device__ __forceinline__ float2 pair_scalar2(float2 r2, float2 nqq, float2 nA, float2 B, const PairParams2& pc,
-                                               float2& e_lj, float2& e_c)
+                                               const EwaldPoly& ep, float2& e_lj, float2& e_c)
 {
     // the hardware reciprocal square root alone: a Newton step on top of it
     // moves the forces' error against FP64 by 1e-8 relative RMS and costs
     // four packed instructions a word
     const float2 rinv = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
     const float2 r2inv = __fmul2_rn(rinv, rinv);
-    const float2 r6inv = __fmul2_rn(__fmul2_rn(r2inv, r2inv), r2inv);
+    const float2 r3inv = __fmul2_rn(rinv, r2inv);
+    const float2 r6inv = __fmul2_rn(r3inv, r3inv);
     // u = (-A/r^6 + B)/r^6 serves the force and, plus B/r^6, the energy
     const float2 u = __fmul2_rn(__ffma2_rn(nA, r6inv, B), r6inv);
     if (ENERGY) e_lj = __ffma2_rn(B, r6inv, u);  // -A/r^12 + 2B/r^6 = -12 E_lj
-    if (FIT == 1)
+    if (FIT != 0)
     {
-        const float2 x = __fmul2_rn(r2, pc.w_scale);
-        if (!ENERGY)
+        float2 s;  // K: 1/r^3 - beta^3 K;  M: t
+        if (FIT == 2)
         {
-            const float2 kp = polyx2(x, kEwaldKP2), kq = polyx2(x, kEwaldKQ2);
-            const float2 K = __fmul2_rn(kp, make_float2(rcp_approx(kq.x), rcp_approx(kq.y)));
-            return __ffma2_rn(nqq, __ffma2_rn(pc.nbeta3, K, __fmul2_rn(rinv, r2inv)), __fmul2_rn(u, r2inv));
+            const float2 q = polyx2(r2, ep.q);
+            s = __ffma2_rn(polyx2(r2, ep.p), make_float2(rcp_approx(q.x), rcp_approx(q.y)), ENERGY ? rinv : r3inv);
         }
-        const float2 mp = polyx2(x, kEwaldMP2), mq = polyx2(x, kEwaldMQ2);
-        const float2 M = __fmul2_rn(mp, make_float2(rcp_approx(mq.x), rcp_approx(mq.y)));
+        else
+        {
+            const float2 x = __fmul2_rn(r2, pc.w_scale);
+            const float2 p = ENERGY ? polyx2(x, kEwaldMP2) : polyx2(x, kEwaldKP2);
+            const float2 q = ENERGY ? polyx2(x, kEwaldMQ2) : polyx2(x, kEwaldKQ2);
+            const float2 k = __fmul2_rn(p, make_float2(rcp_approx(q.x), rcp_approx(q.y)));
+            s = ENERGY ? __ffma2_rn(pc.nbeta, k, rinv) : __ffma2_rn(pc.nbeta3, k, r3inv);
+        }
+        if (!ENERGY) return __ffma2_rn(nqq, s, __fmul2_rn(u, r2inv));
         const float2 wl = __fmul2_rn(r2, pc.nb2_log2e);
         const float2 E = make_float2(ex2_approx(wl.x), ex2_approx(wl.y));
-        const float2 t = __ffma2_rn(pc.nbeta, M, rinv);
-        e_c = __fmul2_rn(nqq, t);
-        return __fmul2_rn(r2inv, __ffma2_rn(nqq, __ffma2_rn(pc.beta_2_sqrtpi, E, t), u));
+        e_c = __fmul2_rn(nqq, s);
+        return __fmul2_rn(r2inv, __ffma2_rn(nqq, __ffma2_rn(pc.beta_2_sqrtpi, E, s), u));
     }
     float c[2], e[2];
     const float rr[2] = {r2.x, r2.y}, ri[2] = {rinv.x, rinv.y}, q[2] = {nqq.x, nqq.y};
@@ -177,6 +192,12 @@ __device__ __forceinline__ float centre_step(int qj, int qi)
     return __int_as_float(((qj - qi + 0x200000) & 0x3fffff) | 0x4b000000) - 10485760.0f;
 }
 
+
+__device__ __forceinline__ void load_rec(const SlotRec* r, float4& pos, int4& aux)
+{
+    pos = r->pos;
+    aux = r->aux;
+}
 
 // Adds to a 64-bit sum in global memory without reading it back (the compiler
 // makes a returning ATOMG of an unused atomicAdd here).
