@@ -407,13 +407,13 @@ __device__ __forceinline__ float3 frac_to_cart(float3 f, const Cell& c)
 // the masks assembled by ballots: about 250 instructions for four candidates,
 // where one candidate a step with two pairs a lane took over 100 for each.
 // The kernel is bound by the instructions it issues (119 M on the 96,000-atom
-// box, 259 M before; loading a step ahead only added some): 378 us to 180
-// there, 110 to 36 on an 8,200-atom box with teams.
-// TEAM = 1: a warp takes a cluster; TEAM = 4: a block of four warps takes one,
-// each a share of its candidates, their results joined in order (boxes with
-// too few clusters to fill the chip with a warp each).
-constexpr int kSearchWarps = 4;
-constexpr int kSearchBlocks = 6;    // resident blocks per SM (5: 183 us on the 96,000-atom box, 6: 180, 7, spilling: 311)
+// box, 259 M before; loading a step ahead only added some): 378 us to 162
+// there, 110 to 33 on an 8,200-atom box with teams.
+// TEAM = 1: a warp takes a cluster; TEAM = 2 or 4: a block of that many warps
+// takes one, each a share of its candidates, their results joined in order
+// (boxes with too few clusters to fill the chip with a warp each).
+constexpr int kSearchResident = 28;  // resident warps per SM (24: 171 us on the 96,000-atom box, 28: 162)
+constexpr int kSearchWaves = 8;      // blocks launched, in waves of the resident ones, at most
 constexpr int kSearchQueue = 256;   // candidates that passed the bounding test, waiting for their decision
 constexpr int kSearchStage = 128;   // table elements a team's warp holds until they are joined
 constexpr float kBorderBand = 1.0e-4f;
@@ -472,15 +472,15 @@ __device__ __forceinline__ int ex_reach(int g, int2 e)
 }
 
 template <int TEAM>
-__global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlocks) k_search(const SearchArgs A)
+__global__ void __launch_bounds__(TEAM * 32, (TEAM > 1 ? 24 : kSearchResident) / TEAM) k_search(const SearchArgs A)
 {
     grid_dep_wait();
     if (A.go && *A.go == 0) return;
-    __shared__ SearchOwn own_all[kSearchWarps];
-    __shared__ int queue_all[kSearchWarps][kSearchQueue];  // surviving candidates {cluster | stencil flags << 28}
-    __shared__ float4 stage_t[TEAM > 1 ? kSearchWarps : 1][TEAM > 1 ? kSearchStage : 1];
-    __shared__ uint2 stage_m[TEAM > 1 ? kSearchWarps : 1][TEAM > 1 ? kSearchStage : 1];
-    __shared__ int team_next, team_count[kSearchWarps];
+    __shared__ SearchOwn own_all[TEAM];
+    __shared__ int queue_all[TEAM][kSearchQueue];  // surviving candidates {cluster | stencil flags << 28}
+    __shared__ float4 stage_t[TEAM][TEAM > 1 ? kSearchStage : 1];
+    __shared__ uint2 stage_m[TEAM][TEAM > 1 ? kSearchStage : 1];
+    __shared__ int team_count[TEAM];
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
     SearchOwn& own = own_all[w];
@@ -489,25 +489,9 @@ __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlock
     const int e_lane = lane >> 3, b_lane = lane & 7;
     unsigned long long elements = 0, listed = 0;
 
-    // clusters are taken from a counter (their tables differ in length)
-    for (;;)
-    {
-        int c = 0;
-        if (TEAM == 1)
-        {
-            if (lane == 0) c = atomicAdd(&A.counters[kCntSearchNext], 1);
-            c = __shfl_sync(0xffffffffu, c, 0);
-        }
-        else
-        {
-            __syncthreads();  // the previous cluster is done with
-            if (threadIdx.x == 0) team_next = atomicAdd(&A.counters[kCntSearchNext], 1);
-            __syncthreads();
-            c = team_next;
-        }
-        if (c >= A.clusters_cap) break;
+    auto cluster = [&](int c) {
         const int sy = A.cl_sys[c];
-        if (!A.need[sy] || c - A.sys[sy].cl_begin >= A.ncl[sy]) continue;
+        if (!A.need[sy] || c - A.sys[sy].cl_begin >= A.ncl[sy]) return;
         const SysDesc& p = A.sys[sy];
         const uint4 ui = A.cl_u[c];
         const int4 qc = A.cl_q[c];
@@ -605,7 +589,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlock
                 if (!__all_sync(0xffffffffu, flags == 3))
                 {
                     unsigned lower = 0;
-#pragma unroll
+    #pragma unroll
                     for (int a = 0; a < kClusterSize; a++) lower |= (own.gid[a] < gb ? 1u : 0u) << a;
                     rule &= ((flags & 1) ? lower : 0u) | ((flags & 2) ? ~lower : 0u);
                 }
@@ -616,7 +600,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlock
                 const float2 ex2 = make_float2(ex, ex), ey2 = make_float2(ey, ey), ez2 = make_float2(ez, ez);
                 unsigned hit = 0;
                 float near = 3.0e38f;
-#pragma unroll
+    #pragma unroll
                 for (int q = 3; q >= 0; q--)
                 {
                     const float2 dx = __fadd2_rn(ex2, reinterpret_cast<const float2*>(own.neg[0])[q]);
@@ -632,7 +616,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlock
                 {
                     // the reference's expression for the pairs that need it
                     const float4 xj = A.slot_x0[slot];
-#pragma unroll 1
+    #pragma unroll 1
                     for (int a = 0; a < kClusterSize; a++)
                     {
                         const float dx = ex + own.neg[0][a], dy = ey + own.neg[1][a], dz = ez + own.neg[2][a];
@@ -653,12 +637,12 @@ __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlock
                 // for all own atoms by the smallest ga - gb + reach (unsigned)
                 const int r = max(reach, ex_reach(gb, ej));
                 unsigned nearest = 0xffffffffu;
-#pragma unroll
+    #pragma unroll
                 for (int a = 0; a < kClusterSize; a++) nearest = min(nearest, (unsigned)(own.gid[a] + (r - gb)));
                 if (__any_sync(0xffffffffu, hit != 0u && r >= 0 && nearest <= 2u * (unsigned)r))
                 {
                     // the lower index's list, scanned only within its range
-#pragma unroll 1
+    #pragma unroll 1
                     for (int a = 0; a < kClusterSize; a++)
                     {
                         const int ga = own.gid[a];
@@ -672,7 +656,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlock
                 }
                 // the four candidates' masks: byte e of ballot a is own atom a's row
                 unsigned row[kClusterSize];
-#pragma unroll
+    #pragma unroll
                 for (int a = 0; a < kClusterSize; a++) row[a] = __ballot_sync(0xffffffffu, hit & (1u << a));
                 const unsigned pick = e_lane | (e_lane + 4) << 4;
                 uint2 m;
@@ -692,8 +676,8 @@ __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlock
                     }
                     else
                     {
-                        stage_t[TEAM > 1 ? w : 0][TEAM > 1 ? at : 0] = t;
-                        stage_m[TEAM > 1 ? w : 0][TEAM > 1 ? at : 0] = m;
+                        stage_t[w][TEAM > 1 ? at : 0] = t;
+                        stage_m[w][TEAM > 1 ? at : 0] = m;
                     }
                     listed += __popc(m.x) + __popc(m.y);
                 }
@@ -729,7 +713,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlock
                     // the run candidate t falls into: the number of runs that end at or before it
                     const int t = t0 + lane;
                     int k = 0;
-#pragma unroll
+    #pragma unroll
                     for (int o = 16; o > 0; o >>= 1)
                         if (__shfl_sync(0xffffffffu, incl, k + o - 1) <= t) k += o;
                     k = min(k, 31);
@@ -798,7 +782,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlock
             if (lane == 0) team_count[w] = count;
             __syncthreads();
             int start = 0, sum = 0, most = 0;
-#pragma unroll
+    #pragma unroll
             for (int v = 0; v < TEAM; v++)
             {
                 const int k = team_count[v];
@@ -826,7 +810,13 @@ __global__ void __launch_bounds__(kSearchWarps * 32, TEAM > 1 ? 4 : kSearchBlock
                 elements += (unsigned long long)min(sum, A.table_cap);
             }
         }
-    }
+    };
+    // one cluster a block, or, a warp a block in a large pool, several
+    // (launch_search)
+    if (TEAM > 1)
+        cluster(blockIdx.x);
+    else
+        for (int c = blockIdx.x; c < A.clusters_cap; c += gridDim.x) cluster(c);
     for (int o = 16; o > 0; o >>= 1) listed += __shfl_xor_sync(0xffffffffu, listed, o);
     if (lane == 0)
     {
@@ -1126,7 +1116,6 @@ __device__ __forceinline__ void reset_list_counters(int* counters)
     counters[kCntWords + 1] = 0;
     counters[kCntPWordsLast] = 0;
     counters[kCntPWordsLast + 1] = 0;
-    counters[kCntSearchNext] = 0;
 }
 
 __global__ void k_reset_list_counters(int* counters)
@@ -1185,7 +1174,6 @@ __global__ void k_sym_begin(int* counters)
     counters[kCntEntries + 1] = 0;
     counters[kCntWords] = 0;
     counters[kCntWords + 1] = 0;
-    counters[kCntSearchNext] = 0;
 }
 
 __global__ void k_init_atom_groups(int n, spgnb_atom_group* nl, int* temp, int max_nb)
@@ -1202,10 +1190,15 @@ __global__ void k_init_atom_groups(int n, spgnb_atom_group* nl, int* temp, int m
 // --------------------------------------------------------------- host side
 
 // The search of the list's clusters (go: the device flag that lets it run,
-// null: always).  A block of four warps per cluster while the chip has room
-// for that many blocks (eight a SM), else a warp per cluster: with fewer
-// clusters than the chip has warps, one warp's walk over a cluster's
-// candidates is the kernel's time.
+// null: always).  A block of four warps per cluster while the chip holds
+// about that many (sixteen an SM), of two up to twice as many, else a warp:
+// with fewer clusters than the chip has warps, one warp's walk over a
+// cluster's candidates is the kernel's time (15,000 atoms: 66 us with a warp,
+// 50 with two; 8,200 atoms 33 with four; 24,000 atoms 75 with a warp, 74 with
+// two, 93 with four).  One-warp blocks leave the distribution to the hardware
+// (162 us on the 96,000-atom box, 180 with four-warp blocks and a counter); in
+// a large pool, whose capacity is mostly parked, a block takes several
+// clusters, so that the launch of a step without a rebuild stays short.
 int launch_search(const spgnb_nl* nl, const int* need, const int* ex_start, const int* ex_list, const int* ex_num,
                   const int* go, int half, const unsigned char* two_sided, cudaStream_t s)
 {
@@ -1240,9 +1233,11 @@ int launch_search(const spgnb_nl* nl, const int* need, const int* ex_start, cons
     a.two_sided_atoms = two_sided;
     const int ccap = nl->clusters_cap, sms = num_sms();
     if (ccap <= sms * 16)
-        launch_dependent(k_search<4>, std::max(1, std::min(ccap, sms * 8)), kSearchWarps * 32, 0, s, a);
+        launch_dependent(k_search<4>, ccap, 4 * 32, 0, s, a);
+    else if (ccap <= sms * 32)
+        launch_dependent(k_search<2>, ccap, 2 * 32, 0, s, a);
     else
-        launch_dependent(k_search<1>, std::max(1, std::min((ccap + kSearchWarps - 1) / kSearchWarps, sms * 8)), kSearchWarps * 32, 0, s, a);
+        launch_dependent(k_search<1>, std::min(ccap, sms * kSearchResident * kSearchWaves), 32, 0, s, a);
     SPGNB_CHECK_LAUNCH("k_search");
     return SPGNB_OK;
 }
