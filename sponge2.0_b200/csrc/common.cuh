@@ -109,7 +109,6 @@ void dfree(T*& p)
 
 // ---------------------------------------------------------------- constants
 constexpr int kClusterSize = 8;       // atoms per cluster
-constexpr int kChunk = 32;            // table elements a search warp stages before writing
 constexpr int kMaxStencil = 192;      // MAX_GRID_NEIGHBORS of neighbor_list.cpp:3
 constexpr int kMaxCellAtoms = 2048;   // hard per-cell capacity of the in-cell sort
 constexpr double kForceScale = 4294967296.0;   // 2^32 per kcal/mol/A

@@ -14,8 +14,8 @@
 // so a step never synchronises with the host):
 //   bin -> scan -> scatter -> in-cell sort -> cluster centres   (clusters)
 //   search  -> per cluster, its neighbour clusters with exact 64-bit masks
-// The force call prunes the tables into per-atom lists (pair.cu); the
-// reference-layout export reads the tables.
+// The force call prunes the tables into per-cluster lists (cluster_pair.cu);
+// the reference-layout export reads the tables.
 #include <math.h>
 #include <string.h>
 
@@ -1165,8 +1165,8 @@ __global__ void k_fill_int(int* __restrict__ p, long long n, int v)
         p[i] = v;
 }
 
-// Before a search that re-makes the last build's tables two-sided: the
-// cluster counter and the table statistics start again.
+// Before a search that re-makes the last build's tables two-sided: the table
+// statistics start again.
 __global__ void k_sym_begin(int* counters)
 {
     grid_dep_wait();

@@ -32,20 +32,6 @@ __device__ __forceinline__ float3 pair_offset(float ex, float ey, float ez, floa
     return make_float3(dx, dy, dz);
 }
 
-// Transpose of an 8x8 bit matrix held as 64 bits, row r in byte r (bit 8r + c
-// moves to bit 8c + r): three rounds of swapping off-diagonal blocks of
-// 1x1, 2x2 and 4x4 bits (H. S. Warren, Hacker's Delight, 2nd ed., section 7-3).
-__device__ __forceinline__ unsigned long long transpose8x8(unsigned long long x)
-{
-    unsigned long long t = (x ^ (x >> 7)) & 0x00AA00AA00AA00AAull;
-    x ^= t ^ (t << 7);
-    t = (x ^ (x >> 14)) & 0x0000CCCC0000CCCCull;
-    x ^= t ^ (t << 14);
-    t = (x ^ (x >> 28)) & 0x00000000F0F0F0F0ull;
-    x ^= t ^ (t << 28);
-    return x;
-}
-
 // ------------------------------------------------ packed FP32x2 pair math
 __device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
 
