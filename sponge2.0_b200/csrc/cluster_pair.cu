@@ -444,6 +444,7 @@ __global__ void __launch_bounds__(32, kPairResident[MODE])
     if (only && !only[sy]) return;
     const ForceParams P = fps ? fps[sy] : p0;
     const PairParams2 pp = pack_params(P);
+    const float2 lead = fit_lead<EN, FIT>(ep);
     const SysDesc& D = sys[sy];
     const Cell qc = D.qcell;
     const int slot0 = D.cl_begin * kClusterSize;
@@ -555,13 +556,16 @@ __global__ void __launch_bounds__(32, kPairResident[MODE])
                     dz = make_float2(ddz[0], ddz[1]);
                 }
                 const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-                const bool inA = (wc & (1u << (kWordMaskShift + 2 * p))) && r2.x < pp.rc2;
-                const bool inB = (wc & (2u << (kWordMaskShift + 2 * p))) && r2.y < pp.rc2;
                 const float4 ab = rows[p * nt + tj];
                 float2 elj, ec;
                 float2 f = pair_scalar2<EN, FIT>(r2, __fmul2_rn(qj, pq), make_float2(ab.x, ab.y),
-                                                 make_float2(ab.z, ab.w), pp, ep, elj, ec);
-                f = make_float2(inA ? f.x : 0.0f, inB ? f.y : 0.0f);
+                                                 make_float2(ab.z, ab.w), pp, ep, lead, elj, ec);
+                const unsigned bitA = 1u << (kWordMaskShift + 2 * p), bitB = 2u << (kWordMaskShift + 2 * p);
+                auto inside = [&](float2 v) {
+                    return make_float2(inside_or_zero(v.x, r2.x, pp.rc2, wc, bitA),
+                                       inside_or_zero(v.y, r2.y, pp.rc2, wc, bitB));
+                };
+                f = inside(f);
                 fx[p] = __ffma2_rn(f, dx, fx[p]);
                 fy[p] = __ffma2_rn(f, dy, fy[p]);
                 fz[p] = __ffma2_rn(f, dz, fz[p]);
@@ -571,8 +575,8 @@ __global__ void __launch_bounds__(32, kPairResident[MODE])
                 const float2 gx = __fmul2_rn(f, dx), gy = __fmul2_rn(f, dy), gz = __fmul2_rn(f, dz);  // the virial's
                 if (EN && !PA)
                 {
-                    acc[0] = __fadd2_rn(acc[0], make_float2(inA ? elj.x : 0.0f, inB ? elj.y : 0.0f));
-                    acc[1] = __fadd2_rn(acc[1], make_float2(inA ? ec.x : 0.0f, inB ? ec.y : 0.0f));
+                    acc[0] = __fadd2_rn(acc[0], inside(elj));
+                    acc[1] = __fadd2_rn(acc[1], inside(ec));
                     acc[2] = __ffma2_rn(gx, dx, acc[2]);
                     acc[3] = __ffma2_rn(gx, dy, acc[3]);
                     acc[4] = __ffma2_rn(gy, dy, acc[4]);
@@ -587,8 +591,7 @@ __global__ void __launch_bounds__(32, kPairResident[MODE])
                     // the word's atoms)
                     const int2 pg = igid[p];
                     const float2 wi = make_float2(pg.x < gj ? 1.0f : 0.0f, pg.y < gj ? 1.0f : 0.0f);
-                    const float2 v[8] = {make_float2(inA ? elj.x : 0.0f, inB ? elj.y : 0.0f),
-                                         make_float2(inA ? ec.x : 0.0f, inB ? ec.y : 0.0f),
+                    const float2 v[8] = {inside(elj), inside(ec),
                                          __fmul2_rn(gx, dx), __fmul2_rn(gx, dy), __fmul2_rn(gy, dy),
                                          __fmul2_rn(gx, dz), __fmul2_rn(gy, dz), __fmul2_rn(gz, dz)};
 #pragma unroll
@@ -947,9 +950,10 @@ EwaldPoly scaled_fit(const ForceParams& f, bool energy)
 {
     EwaldPoly e;
     const double b = f.beta, w = b * b / (double)SPGNB_EWALD_W_MAX;
-    double np = energy ? -b : -b * b * b, nq = 1.0;
+    double nq = 1.0 / (w * w * w * w * w), np = (energy ? -b : -b * b * b) * nq;
     for (int k = 0; k < 6; k++, np *= w, nq *= w)
     {
+        // divided by w^5: the denominator stays monic
         const float p = (float)((energy ? kEwaldMPHost[k] : kEwaldKPHost[k]) * np);
         const float q = (float)((energy ? kEwaldMQHost[k] : kEwaldKQHost[k]) * nq);
         e.p[k] = make_float2(p, p);
@@ -997,13 +1001,15 @@ int launch_pair_t(const ForceInputs& in, bool tri, cudaStream_t s)
     return tri ? launch_pair<M, F, true>(in, s) : launch_pair<M, F, false>(in, s);
 }
 
-// FIT 2, the fits scaled to the call's one system, or 1 for several systems;
-// 0 outside the fits' range.
+// FIT 2, the fits scaled to the call's one system, or 1 for several systems
+// and for an Ewald parameter so small (beta below 0.0035 / A, or none) that the
+// scaled coefficients, up to beta^-10, would leave FP32's range; 0 outside the
+// fits' range.
 template <int M>
 int launch_pair_ft(const ForceInputs& in, bool tri, cudaStream_t s)
 {
     if (!in.fit) return launch_pair_t<M, 0>(in, tri, s);
-    return in.d_fps ? launch_pair_t<M, 1>(in, tri, s) : launch_pair_t<M, 2>(in, tri, s);
+    return in.d_fps || in.p0.w_scale < 1e-6f ? launch_pair_t<M, 1>(in, tri, s) : launch_pair_t<M, 2>(in, tri, s);
 }
 
 }  // namespace

@@ -113,6 +113,10 @@ def main():
     mp, mq, merr = ratfit(M)
     kp2, kq2, kerr2 = minimax(K, DEG, DEG)
     mp2, mq2, merr2 = minimax(M, DEG, DEG)
+    # the packed kernel's denominators are monic: their first step is an
+    # addition with one constant operand
+    kp2, kq2 = kp2 / kq2[-1], kq2 / kq2[-1]
+    mp2, mq2 = mp2 / mq2[-1], mq2 / mq2[-1]
     fmt = lambda a: ", ".join(f"{float(v):.9e}f" for v in a)
     print("// Generated by gen_ewald_fit.py -- do not edit.")
     print(f"// K(w) max abs error {kerr:.2e} (K(0)=0.752), M(w) max abs error {merr:.2e} (M(0)=1.128),")

@@ -48,13 +48,40 @@ enum PackedConst
 constexpr float kLjEnergyScale = -1.0f / 12.0f;
 constexpr float kCoulombEnergyScale = -1.0f;
 
-template <int N>
-__device__ __forceinline__ float2 polyx2(float2 x, const float2 (&c)[N])
+// Degree-5 polynomials by Horner's rule.  The packed instruction takes one
+// constant operand, so the numerator's leading coefficient comes in a
+// register (lead) and the denominator is monic.
+__device__ __forceinline__ float2 polyx2(float2 x, float2 lead, const float2 (&c)[6])
 {
-    float2 p = c[N - 1];
-#pragma unroll
-    for (int k = N - 2; k >= 0; k--) p = __ffma2_rn(p, x, c[k]);
-    return p;
+    float2 p = __ffma2_rn(lead, x, c[4]);
+    p = __ffma2_rn(p, x, c[3]);
+    p = __ffma2_rn(p, x, c[2]);
+    p = __ffma2_rn(p, x, c[1]);
+    return __ffma2_rn(p, x, c[0]);
+}
+
+__device__ __forceinline__ float2 polyx2_monic(float2 x, const float2 (&c)[6])
+{
+    float2 p = __fadd2_rn(x, c[4]);
+    p = __ffma2_rn(p, x, c[3]);
+    p = __ffma2_rn(p, x, c[2]);
+    p = __ffma2_rn(p, x, c[1]);
+    return __ffma2_rn(p, x, c[0]);
+}
+
+// v where the list word pairs the atom (w & bit) and r2 is inside the cutoff,
+// else 0: the bit test, the comparison and their conjunction in two
+// instructions (a logic operation with a predicate result).
+__device__ __forceinline__ float inside_or_zero(float v, float r2, float rc2, unsigned w, unsigned bit)
+{
+    float o;
+    asm("{\n\t.reg .pred p, q;\n\t.reg .b32 d;\n\t"
+        "setp.lt.f32 q, %2, %3;\n\t"
+        "lop3.and.b32 d|p, %4, %5, 0, 0xC0, q;\n\t"
+        "selp.f32 %0, %1, 0f00000000, p;\n\t}"
+        : "=f"(o)
+        : "f"(v), "f"(r2), "f"(rc2), "r"(w), "r"(bit));
+    return o;
 }
 
 __device__ __forceinline__ float ex2_approx(float x)
@@ -82,7 +109,7 @@ __device__ __forceinline__ float rcp_approx(float x)
     return y;
 }
 
-// A fit's numerator and denominator as polynomials in r^2, (c, c) pairs.
+// A fit's numerator and (monic) denominator as polynomials in r^2, (c, c) pairs.
 struct EwaldPoly
 {
     float2 p[6], q[6];
@@ -119,9 +146,20 @@ __device__ __forceinline__ PairParams2 pack_params(const ForceParams& pc)
 // FIT 1: the fits in w / W_MAX; FIT 2: the same fits as polynomials in r^2
 // with -beta^3 (K) or -beta (M) in the numerator, ep, made for the one system
 // of a call: two packed instructions fewer a pair.  FIT 0: erfc.
+// lead: the numerator's leading coefficient (fit_lead).
+template <bool ENERGY, int FIT>
+__device__ __forceinline__ float2 fit_lead(const EwaldPoly& ep)
+{
+    float2 l = FIT == 2 ? ep.p[5] : (ENERGY ? kEwaldMP2[5] : kEwaldKP2[5]);
+    // opaque, so that it stays in registers over the list instead of being
+    // moved there for every pair
+    asm volatile("" : "+f"(l.x), "+f"(l.y));
+    return l;
+}
+
 template <bool ENERGY, int FIT>
 __device__ __forceinline__ float2 pair_scalar2(float2 r2, float2 nqq, float2 nA, float2 B, const PairParams2& pc,
-                                               const EwaldPoly& ep, float2& e_lj, float2& e_c)
+                                               const EwaldPoly& ep, float2 lead, float2& e_lj, float2& e_c)
 {
     // the hardware reciprocal square root alone: a Newton step on top of it
     // moves the forces' error against FP64 by 1e-8 relative RMS and costs
@@ -138,14 +176,14 @@ __device__ __forceinline__ float2 pair_scalar2(float2 r2, float2 nqq, float2 nA,
         float2 s;  // K: 1/r^3 - beta^3 K;  M: t
         if (FIT == 2)
         {
-            const float2 q = polyx2(r2, ep.q);
-            s = __ffma2_rn(polyx2(r2, ep.p), make_float2(rcp_approx(q.x), rcp_approx(q.y)), ENERGY ? rinv : r3inv);
+            const float2 q = polyx2_monic(r2, ep.q);
+            s = __ffma2_rn(polyx2(r2, lead, ep.p), make_float2(rcp_approx(q.x), rcp_approx(q.y)), ENERGY ? rinv : r3inv);
         }
         else
         {
             const float2 x = __fmul2_rn(r2, pc.w_scale);
-            const float2 p = ENERGY ? polyx2(x, kEwaldMP2) : polyx2(x, kEwaldKP2);
-            const float2 q = ENERGY ? polyx2(x, kEwaldMQ2) : polyx2(x, kEwaldKQ2);
+            const float2 p = ENERGY ? polyx2(x, lead, kEwaldMP2) : polyx2(x, lead, kEwaldKP2);
+            const float2 q = ENERGY ? polyx2_monic(x, kEwaldMQ2) : polyx2_monic(x, kEwaldKQ2);
             const float2 k = __fmul2_rn(p, make_float2(rcp_approx(q.x), rcp_approx(q.y)));
             s = ENERGY ? __ffma2_rn(pc.nbeta, k, rinv) : __ffma2_rn(pc.nbeta3, k, r3inv);
         }

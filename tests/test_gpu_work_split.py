@@ -75,3 +75,20 @@ def test_split_lists_and_forces(torch_cuda, oracle, name):
             # the per-atom arrays hold the same pairs: N FP32 values summed
             assert abs(p.atom_energy.double().sum().item() - tot[0] - tot[1]) <= 1e-6 * scale
             assert np.abs(p.atom_virial.double().sum(0).cpu().numpy() - tot[2:]).max() <= 1e-6 * np.abs(tot[2:]).max()
+
+
+@pytest.mark.parametrize("beta", [0.0, 0.002, 0.01, 0.2, 0.34, 0.5])
+def test_ewald_fit_routes(torch_cuda, oracle, beta):
+    """The pair function's fits over the Ewald parameters that take each form:
+    in w (none, tiny), scaled to the system, and erfc past the fits' range."""
+    from dataclasses import replace
+    from spgnb.engine import PlainPath
+    s = replace(_water(700, 8.0, 53, n_solute=40), beta=beta)
+    p = PlainPath(s, export_atom_groups=True)
+    counts, lists = p.nl.host_atom_groups()
+    ref = oracle.pair_force(s, counts, lists, per_atom=False)
+    for energy in (False, True):
+        frc = p.force(need_energy=energy, need_virial=energy, per_atom=False).cpu().numpy()
+        assert rel_rms(frc, ref["frc"]) <= FORCE_REL_RMS_TOL
+    tot = p.lj.totals()
+    assert abs(tot[1] - ref["e_coul"]) <= 1e-5 * (abs(ref["e_lj"]) + abs(ref["e_coul"]))
