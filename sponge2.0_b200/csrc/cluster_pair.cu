@@ -399,7 +399,8 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
 // shared memory rings 91 and 1,364).  Partner sums go out by RED (red_add):
 // the ATOMG that atomicAdd becomes here waits for an answer, and with it and
 // a test per component instead of one per word the two boxes took 103 and
-// 1,548, the per-atom mode 217 instead of 151.
+// 1,548, the per-atom mode 217 instead of 151.  With 32-byte records and the
+// fits as they are now (pairfn.cuh) the three take 71.5, 1,131 and 146.
 //
 // Each pair is evaluated once; a lane holds all 8 atoms, the partner's force
 // (summed over the 8 in a fixed order) goes to its int64 fixed-point
