@@ -1464,10 +1464,15 @@ SysDesc make_desc(const SysHost& sh, float skin_permit)
     d.frac_norm[1] = sqrtf(d.rcell.a22 * d.rcell.a22 + d.rcell.a32 * d.rcell.a32);
     d.frac_norm[2] = fabsf(d.rcell.a33);
     // a pair beyond half a box in a fractional coordinate f has another image
-    // at 1 - f; past this bound on f that image could come within the list
-    // radius, and the pair needs its own
+    // at 1 - f; past this bound on f that image could come within the cutoff
+    // before the next build, and the pair needs its own.  The margin is a skin
+    // past the list radius, so atoms may drift by a whole skin each, twice what
+    // keeps the list complete: with rebuilds at a fixed interval, or a skin
+    // permit above a half, a listed pair is still evaluated at the image the
+    // reference takes.
+    const float slack = sh.skin * fmaxf(1.0f, 2.0f * skin_permit - 1.0f) + 0.01f;
     for (int k = 0; k < 3; k++)
-        d.image_bound[k] = fmaxf(0.49f, 1.0f - 1e-4f - (d.list_radius + 0.01f) * d.frac_norm[k]);
+        d.image_bound[k] = fmaxf(0.49f, 1.0f - 1e-4f - (d.list_radius + slack) * d.frac_norm[k]);
     d.Nx = sh.dims[0];
     d.Ny = sh.dims[1];
     d.Nz = sh.dims[2];
