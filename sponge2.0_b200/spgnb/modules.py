@@ -332,14 +332,14 @@ class SOLVENT_LENNARD_JONES:
         arrays = [_ptr(t) for t in (d_res_start, crd, charge, frc, atom_energy, atom_lj_virial,
                                     atom_direct_pme_energy)]
         cells = LTMatrix3.of(cell), LTMatrix3.of(rcell)
+        numbers = int(atom_numbers), int(residue_numbers)
+        beta, energy, virial = float(pme_beta), int(need_atom_energy), int(need_virial)
         if isinstance(nl, NEIGHBOR_LIST) and nl.handle is not None:
             return  # over an spgnb list the LJ module's call evaluates the waters too
         _bind_stream()
-        check(lib().spgnb_solvent_pme_direct_force(self.handle, int(atom_numbers), int(residue_numbers),
-                                                   *arrays[:4], *cells, None,
-                                                   None if isinstance(nl, NEIGHBOR_LIST) else int(nl),
-                                                   float(pme_beta), int(need_atom_energy), arrays[4],
-                                                   int(need_virial), arrays[5], arrays[6]))
+        check(lib().spgnb_solvent_pme_direct_force(self.handle, *numbers, *arrays[:4], *cells, None,
+                                                   None if isinstance(nl, NEIGHBOR_LIST) else int(nl), beta, energy,
+                                                   arrays[4], virial, arrays[5], arrays[6]))
 
     def Clear(self):
         if self.handle is not None:
