@@ -534,15 +534,16 @@ int spgnb_batch_stats(spgnb_batch* b, long long* steps, long long* rebuilds, lon
 /* Picks the launch configuration with the fastest step for this batch by
  * timing a few steps of each candidate, one setting after the other (the
  * systems advance meanwhile): the prune buffer (up to the one the lists were
- * sized for), the force kernel's resident blocks per SM, the pruning
+ * sized for), the force kernel's resident warps per SM, the pruning
  * kernel's blocks per SM and the steps per captured graph.  Results are the
  * same for every choice; only the time differs. */
 int spgnb_batch_autotune(spgnb_batch* b, int steps_per_candidate, float* chosen_buffer);
 typedef struct
 {
     float prune_buffer;         /* A */
-    int pair_blocks_per_sm;     /* force kernel, 0 = as many as are resident */
-    int prune_blocks_per_sm;    /* pruning kernel */
+    int pair_blocks_per_sm;     /* force kernel: groups of four one-warp blocks held resident on an SM
+                                   (by the shared memory each block asks for), 0 = as many as fit */
+    int prune_blocks_per_sm;    /* pruning kernel: its grid, in blocks of eight warps per SM */
     int steps_per_graph;
     float ms_per_step;          /* of the chosen configuration, 0 before any tuning */
 } spgnb_batch_tuning;

@@ -963,6 +963,26 @@ EwaldPoly scaled_fit(const ForceParams& f, bool energy)
     return e;
 }
 
+// The dynamic shared memory that leaves `blocks` blocks of this kernel
+// resident on an SM: an equal share of the SM's, less the kernel's static
+// memory and what the runtime reserves for each block.  0 when they fit
+// anyhow.
+size_t smem_for_resident(const void* kernel, long long blocks)
+{
+    int dev = 0, per_sm = 0, reserved = 0;
+    cudaFuncAttributes attr{};
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
+        cudaFuncGetAttributes(&attr, kernel) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return 0;
+    }
+    const long long own = (long long)attr.sharedSizeBytes + reserved;
+    return (size_t)std::max(0LL, (per_sm / blocks & ~127LL) - own);  // allocated in units of 128 bytes
+}
+
 template <int M, int F, bool T>
 int launch_pair(const ForceInputs& in, cudaStream_t s)
 {
@@ -970,10 +990,10 @@ int launch_pair(const ForceInputs& in, cudaStream_t s)
     const EwaldPoly ep = F == 2 ? scaled_fit(in.p0, M >= 1) : EwaldPoly{};
     const int mt = in.max_types > 0 ? in.max_types : in.p0.n_types;
     size_t smem = sizeof(float4) * std::max(4 * mt, 2 * kSumRow);
-    // the blocks-per-SM setting counts blocks of four warps: it holds the
-    // resident ones down by the shared memory each asks for
+    // the setting counts groups of four one-warp blocks: it holds the resident
+    // ones down by the shared memory each asks for
     if (in.pair_blocks_per_sm > 0)
-        smem = std::max(smem, (size_t)(220 * 1024 / (4 * in.pair_blocks_per_sm)) & ~(size_t)127);
+        smem = std::max(smem, smem_for_resident((const void*)k_pair8<M, F, T>, 4LL * in.pair_blocks_per_sm));
     // Each cluster's list in 2^shift parts, as many as keep the items within
     // one and a half times the warps the chip holds.  With fewer clusters than
     // warps the kernel's time is one warp's walk over a list: the 6,480-atom

@@ -517,7 +517,7 @@ struct ForceInputs
     long long* totals = nullptr;       // 8 fixed-point sums per system (mode >= 1)
     const int* only = nullptr;         // per-system flags: evaluate these systems only (null: all)
     int mode = 0;                      // 0 forces, 1 + totals, 2 + per-atom outputs
-    int pair_blocks_per_sm = 0;        // force kernel grid: 0 = as many as are resident
+    int pair_blocks_per_sm = 0;        // force kernel: resident warps per SM in fours, 0 = as many as fit
     int prune_blocks_per_sm = 0;       // pruning kernel grid: 0 = 5
     OwnerMap om{nullptr, 0, 3};
     PerAtomOut pa{nullptr, nullptr, nullptr, nullptr};

@@ -34,3 +34,22 @@ def torch_cuda():
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     return torch
+
+
+def kernel_launches(torch, fn):
+    """The GPU kernels fn() runs, in order: {name, grid, block, shared} each."""
+    import json
+    import tempfile
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    with tempfile.TemporaryDirectory() as d:
+        path = os.path.join(d, "trace.json")
+        prof.export_chrome_trace(path)
+        with open(path) as f:
+            events = json.load(f)["traceEvents"]
+    kernels = sorted((e for e in events if e.get("cat") == "kernel"), key=lambda e: e["ts"])
+    return [{"name": e["name"], "grid": e["args"]["grid"], "block": e["args"]["block"],
+             "shared": e["args"]["shared memory"]} for e in kernels]
