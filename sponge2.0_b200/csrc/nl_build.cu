@@ -1463,16 +1463,21 @@ SysDesc make_desc(const SysHost& sh, float skin_permit)
     d.frac_norm[0] = sqrtf(d.rcell.a11 * d.rcell.a11 + d.rcell.a21 * d.rcell.a21 + d.rcell.a31 * d.rcell.a31);
     d.frac_norm[1] = sqrtf(d.rcell.a22 * d.rcell.a22 + d.rcell.a32 * d.rcell.a32);
     d.frac_norm[2] = fabsf(d.rcell.a33);
-    // a pair beyond half a box in a fractional coordinate f has another image
-    // at 1 - f; past this bound on f that image could come within the cutoff
-    // before the next build, and the pair needs its own.  The margin is a skin
-    // past the list radius, so atoms may drift by a whole skin each, twice what
-    // keeps the list complete: with rebuilds at a fixed interval, or a skin
-    // permit above a half, a listed pair is still evaluated at the image the
-    // reference takes.
-    const float slack = sh.skin * fmaxf(1.0f, 2.0f * skin_permit - 1.0f) + 0.01f;
+    // A pair beyond half a box in a fractional coordinate f has another image
+    // at 1 - f; past this bound on f that image could be within the list
+    // radius, and the pair needs its own.  It must also stay out of the cutoff
+    // until the next build, and a listed pair's other image is at least a box
+    // length less the list radius away: with a box of two radii and a skin,
+    // atoms may drift by a whole skin each, twice what keeps the list complete
+    // (further with a skin permit above one), before a pair is evaluated at
+    // another image than the reference's.  A smaller box takes no pair past
+    // 0.49 at one image.
+    const float drift = sh.skin * fmaxf(1.0f, 2.0f * skin_permit - 1.0f);
     for (int k = 0; k < 3; k++)
-        d.image_bound[k] = fmaxf(0.49f, 1.0f - 1e-4f - (d.list_radius + slack) * d.frac_norm[k]);
+    {
+        const bool roomy = (d.list_radius + 0.5f * drift) * d.frac_norm[k] < 0.5f;
+        d.image_bound[k] = roomy ? 1.0f - 1e-4f - (d.list_radius + 0.01f) * d.frac_norm[k] : 0.49f;
+    }
     d.Nx = sh.dims[0];
     d.Ny = sh.dims[1];
     d.Nz = sh.dims[2];
