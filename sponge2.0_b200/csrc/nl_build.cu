@@ -415,7 +415,11 @@ __device__ __forceinline__ float3 frac_to_cart(float3 f, const Cell& c)
 constexpr int kSearchResident = 28;  // resident warps per SM (24: 171 us on the 96,000-atom box, 28: 162)
 constexpr int kSearchWaves = 8;      // blocks launched, in waves of the resident ones, at most
 constexpr int kSearchQueue = 256;   // candidates that passed the bounding test, waiting for their decision
-constexpr int kSearchStage = 128;   // table elements a team's warp holds until they are joined
+// table elements a team's warp holds until they are joined; a share that holds
+// more is searched a second time, straight to the table (at 12 A about a tenth
+// of the clusters of 17,000 to 28,000 atoms have one; with the whole cluster
+// searched again by one warp instead, a build of 21,000 atoms took 257 us, 214 so)
+constexpr int kSearchStage = 128;
 constexpr float kBorderBand = 1.0e-4f;
 
 __device__ bool excluded_scan(int glo, int ghi, const int* __restrict__ ex_start, const int* __restrict__ ex_list,
@@ -543,8 +547,9 @@ __global__ void __launch_bounds__(TEAM * 32, (TEAM > 1 ? 24 : kSearchResident) /
         };
 
         // The elements of candidates [lo, hi) of the flattened runs, to the
-        // table (direct) or to this warp's staging; returns their number.
-        auto search = [&](int lo, int hi, bool direct) -> int {
+        // table from its element `start` on (direct) or to this warp's
+        // staging; returns their number.
+        auto search = [&](int lo, int hi, bool direct, int start) -> int {
             int written = 0, queued = 0;
             // four queued candidates (fewer at the end), one neighbour atom a lane
             auto decide = [&](int q0) {
@@ -664,7 +669,7 @@ __global__ void __launch_bounds__(TEAM * 32, (TEAM > 1 ? 24 : kSearchResident) /
                 m.y = __byte_perm(__byte_perm(row[4], row[5], pick), __byte_perm(row[6], row[7], pick), 0x5410);
                 const bool lead = b_lane == 0 && (m.x | m.y) != 0u;
                 const unsigned leads = __ballot_sync(0xffffffffu, lead);
-                const int at = written + __popc(leads & below);
+                const int at = start + written + __popc(leads & below);
                 const int cap = direct ? A.table_cap : kSearchStage;
                 if (lead && at < cap)
                 {
@@ -759,7 +764,7 @@ __global__ void __launch_bounds__(TEAM * 32, (TEAM > 1 ? 24 : kSearchResident) /
 
         if (TEAM == 1)
         {
-            const int written = search(0, 0x7fffffff, true);
+            const int written = search(0, 0x7fffffff, true, 0);
             if (lane == 0)
             {
                 if (written > A.table_cap) atomicOr(&A.counters[kCntOverflow], kOvfPairs);
@@ -777,24 +782,25 @@ __global__ void __launch_bounds__(TEAM * 32, (TEAM > 1 ? 24 : kSearchResident) /
                 load_run(rb + lane, first, n, flags);
                 all += __reduce_add_sync(0xffffffffu, n);
             }
+            const int lo = (int)((long long)all * w / TEAM), hi = (int)((long long)all * (w + 1) / TEAM);
             const unsigned long long before = listed;
-            const int count = search((int)((long long)all * w / TEAM), (int)((long long)all * (w + 1) / TEAM), false);
+            const int count = search(lo, hi, false, 0);
             if (lane == 0) team_count[w] = count;
             __syncthreads();
-            int start = 0, sum = 0, most = 0;
+            int start = 0, sum = 0;
     #pragma unroll
             for (int v = 0; v < TEAM; v++)
             {
                 const int k = team_count[v];
                 if (v < w) start += k;
                 sum += k;
-                most = max(most, k);
             }
-            if (most > kSearchStage)
+            if (count > kSearchStage)
             {
-                // a share that does not fit its staging: one warp for all
+                // a share that does not fit its staging is searched again,
+                // now that its place in the table is known
                 listed = before;
-                if (w == 0) sum = search(0, 0x7fffffff, true);
+                search(lo, hi, true, start);
             }
             else
                 for (int k = lane; k < count; k += 32)
@@ -1195,7 +1201,11 @@ __global__ void k_init_atom_groups(int n, spgnb_atom_group* nl, int* temp, int m
 // with fewer clusters than the chip has warps, one warp's walk over a
 // cluster's candidates is the kernel's time (15,000 atoms: 66 us with a warp,
 // 50 with two; 8,200 atoms 33 with four; 24,000 atoms 75 with a warp, 74 with
-// two, 93 with four).  One-warp blocks leave the distribution to the hardware
+// two, 93 with four).  Two-sided tables hold twice the elements, more than two
+// warps' shares can stage at the longer cutoffs: a warp each from sixteen an SM
+// on (a build with a two-sided search and dH/dlambda on 21,200 atoms at 12 A:
+// 792 us with two warps, 553 with one; 15,200 atoms at 8 A: 273 and 236).
+// One-warp blocks leave the distribution to the hardware
 // (162 us on the 96,000-atom box, 180 with four-warp blocks and a counter); in
 // a large pool, whose capacity is mostly parked, a block takes several
 // clusters, so that the launch of a step without a rebuild stays short.
@@ -1234,7 +1244,7 @@ int launch_search(const spgnb_nl* nl, const int* need, const int* ex_start, cons
     const int ccap = nl->clusters_cap, sms = num_sms();
     if (ccap <= sms * 16)
         launch_dependent(k_search<4>, ccap, 4 * 32, 0, s, a);
-    else if (ccap <= sms * 32)
+    else if (half && ccap <= sms * 32)
         launch_dependent(k_search<2>, ccap, 2 * 32, 0, s, a);
     else
         launch_dependent(k_search<1>, std::min(ccap, sms * kSearchResident * kSearchWaves), 32, 0, s, a);
