@@ -1658,7 +1658,7 @@ int spgnb_batch_autotune(spgnb_batch* b, int steps_per_candidate, float* chosen_
     }, buffers);
     if (!st)
     {
-        // the force kernel's resident blocks per SM (0: all that fit)
+        // the force kernel's resident warps per SM, in fours (0: all that fit)
         const std::vector<int> pair_bps = {0, 3, 2};
         best_ms = 1e30f;
         tune([&](int c) { b->pair_bps = c; return true; }, pair_bps);

@@ -407,7 +407,10 @@ __global__ void __launch_bounds__(kPruneWarps * 32)
 // accumulator by one atomic add per component and word, and the cluster's
 // forces are summed over the lanes in FP64 in a fixed order and added the same
 // way.  Integer addition does not depend on order, so the forces are bitwise
-// reproducible; the finishing pass converts them.
+// reproducible; the finishing pass converts them.  A lane's FP32 share depends
+// on the parts a list is split into, and those, for one system, on the SM
+// count, the mode and the list's capacity in clusters (launch_pair): one
+// system's last bits can differ between chips, several systems' not.
 //
 // MODE 0: forces.  MODE 1: + energy and virial totals.  MODE 2: + per-atom
 // energy and virial: a pair's terms belong to its owner, the atom with the
@@ -667,7 +670,10 @@ __global__ void __launch_bounds__(32, kPairResident[MODE])
     else if (EN && !PA)
     {
         // each pair once; the virial is -g (x) d, its symmetric
-        // off-diagonal terms (xy + yx etc.) twice the one accumulated
+        // off-diagonal terms (xy + yx etc.) twice the one accumulated.  Eight
+        // adds a list on one line: on the 1.0 M-atom box, where 146,000 lists
+        // meet there, a force call with totals takes 1,682 us (2,065 with the
+        // persistent warps that added theirs once at the end)
         const int q = lane >> 2;
         const double sc = q == 0 ? (double)kLjEnergyScale
                                  : (q == 1 ? (double)kCoulombEnergyScale
@@ -1024,8 +1030,10 @@ int launch_pair_t(const ForceInputs& in, bool tri, cudaStream_t s)
 
 // FIT 2, the fits scaled to the call's one system, or 1 for several systems
 // and for an Ewald parameter so small (beta below 0.0035 / A, or none) that the
-// scaled coefficients, up to beta^-10, would leave FP32's range; 0 outside the
-// fits' range.
+// scaled coefficients, up to beta^-10, would leave FP32's range (at a w_scale
+// of 1e-6 the denominator reaches 7.3e30 and its flushed reciprocal 1.4e-31:
+// lowered by a factor of 20 or more it would leave the normal range); 0 outside the fits'
+// range.
 template <int M>
 int launch_pair_ft(const ForceInputs& in, bool tri, cudaStream_t s)
 {

@@ -353,9 +353,9 @@ struct spgnb_nl
     // pruned per-cluster partner lists (the half list: partners in clusters
     // J > I, and within I the pairs a < b), list_cap words reserved per
     // cluster: {partner slot | atom mask << 22 | image flag << 30}, padded to
-    // 32-word windows; the length at d_pcount[8c] (a cluster near the start
-    // of a periodic box can hold nearly its whole neighbourhood, so the
-    // reserve is sized for that)
+    // 32-word windows; the length at d_pcount[8c], with bit 30 set when some
+    // word has its image flag set (a cluster near the start of a periodic box
+    // can hold nearly its whole neighbourhood, so the reserve is sized for that)
     unsigned* d_pwords = nullptr;
     int* d_pcount = nullptr;
     long long* d_facc = nullptr;  // per slot: the half-list kernel's int64 force sums (3), cleared after use

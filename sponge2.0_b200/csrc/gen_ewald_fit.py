@@ -14,9 +14,9 @@ in double: for the scalar kernels by iteratively reweighted linear least
 squares on the relative error (Loeb's method); for the packed cluster-pair
 kernel by the same linearisation with Lawson's weights, which drive the
 largest absolute error down (minimax: 7e-9 for K, 1e-9 for M, below what FP32
-resolves).  Degrees (4,5) would save the packed kernel an instruction, but
-their 6e-8 is one-sided over whole ranges of r and moved the forces' error
-against 64 bits from 8e-7 to 1.0e-6 relative RMS.
+resolves), scaled to monic denominators.  Degrees (4,5) would save the packed
+kernel an instruction, but their 6e-8 is one-sided over whole ranges of r and
+moved the forces' error against 64 bits from 8e-7 to 1.0e-6 relative RMS.
 W_MAX = 12.25 covers beta*rc <= 3.5, i.e. a direct-space
 tolerance down to ~1e-7 at rc = 10.  Run from this directory:
 ``python gen_ewald_fit.py > ewald_fit.h``.
@@ -102,6 +102,9 @@ def minimax(f, m, n, iters=60):
             lawson = lawson * (err / err.max() + 1e-3) ** 0.5
             lawson /= lawson.max()
     _, p, q = best
+    # the packed kernel's denominators are monic: their first step is an
+    # addition with one constant operand
+    p, q = p / q[-1], q / q[-1]
     w = np.linspace(0, W_MAX, 200001)
     xf = (w / W_MAX).astype(np.float32)
     r = (horner32(p, xf) * (np.float32(1) / horner32(q, xf))).astype(np.float64)
@@ -113,10 +116,6 @@ def main():
     mp, mq, merr = ratfit(M)
     kp2, kq2, kerr2 = minimax(K, DEG, DEG)
     mp2, mq2, merr2 = minimax(M, DEG, DEG)
-    # the packed kernel's denominators are monic: their first step is an
-    # addition with one constant operand
-    kp2, kq2 = kp2 / kq2[-1], kq2 / kq2[-1]
-    mp2, mq2 = mp2 / mq2[-1], mq2 / mq2[-1]
     fmt = lambda a: ", ".join(f"{float(v):.9e}f" for v in a)
     print("// Generated by gen_ewald_fit.py -- do not edit.")
     print(f"// K(w) max abs error {kerr:.2e} (K(0)=0.752), M(w) max abs error {merr:.2e} (M(0)=1.128),")

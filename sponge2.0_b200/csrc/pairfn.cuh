@@ -92,9 +92,12 @@ __device__ __forceinline__ float ex2_approx(float x)
 }
 
 // The hardware approximations with subnormals flushed (PTX rsqrt.approx.ftz,
-// rcp.approx.ftz): r^2 of a listed pair and the fits' denominators (>= 1)
-// are far from the subnormal range, so the range handling of rsqrtf and
-// __fdividef is not needed.
+// rcp.approx.ftz), without the range handling of rsqrtf and __fdividef: r^2
+// of a listed pair is far from the subnormal range.  So are the fits' monic
+// denominators and their reciprocals: in w they lie between 0.028 and 7.3, in
+// r^2 they are divided by the fifth power of the scale of w, which the choice
+// between the two forms keeps at 1e-6 or more (launch_pair_ft): 7.3e30 at
+// most, its reciprocal 1.4e-31.
 __device__ __forceinline__ float rsqrt_approx(float x)
 {
     float y;
