@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(32, kPairResident[MODE])
     {
         // each pair once; the virial is -g (x) d, its symmetric
         // off-diagonal terms (xy + yx etc.) twice the one accumulated.  Eight
-        // adds a list on one line: on the 1.0 M-atom box, where 146,000 lists
+        // adds a list on one line: on the 1.0 M-atom box, where 137,000 lists
         // meet there, a force call with totals takes 1,682 us (2,065 with the
         // persistent warps that added theirs once at the end)
         const int q = lane >> 2;

@@ -37,7 +37,9 @@ def torch_cuda():
 
 
 def kernel_launches(torch, fn):
-    """The GPU kernels fn() runs, in order: {name, grid, block, shared} each."""
+    """The GPU kernels fn() runs, in order: {name, grid, block, shared} each.
+    For a process of its own (in_fresh_process): the tracer loses the first
+    kernels of a profile late in a long test run."""
     import json
     import tempfile
     from torch.profiler import ProfilerActivity, profile
@@ -53,3 +55,14 @@ def kernel_launches(torch, fn):
     kernels = sorted((e for e in events if e.get("cat") == "kernel"), key=lambda e: e["ts"])
     return [{"name": e["name"], "grid": e["args"]["grid"], "block": e["args"]["block"],
              "shared": e["args"]["shared memory"]} for e in kernels]
+
+
+def in_fresh_process(module, function):
+    """What the test module's function returns (JSON values) in a new process."""
+    import json
+    code = (f"import conftest, json, {module}\n"
+            f"print('RESULT ' + json.dumps({module}.{function}()))")
+    r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.abspath(__file__)),
+                       capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+    return json.loads(r.stdout.split("RESULT ", 1)[1])

@@ -9,7 +9,7 @@ a rule that moves fails here instead of leaving a form untested.
 import numpy as np
 import pytest
 
-from conftest import kernel_launches, rel_rms
+from conftest import in_fresh_process, kernel_launches, rel_rms
 
 pytestmark = pytest.mark.gpu
 
@@ -70,25 +70,43 @@ def _split(launches):
     return parts, one["k_search"]["block"][0] // 32, int(one["k_prune8"]["name"].split("k_prune8<")[1][0])
 
 
-@pytest.mark.parametrize("name", list(CASES))
-def test_split_lists_and_forces(torch_cuda, oracle, name):
+def _path(s, **kw):
     from spgnb.engine import PlainPath
-    make, *split = CASES[name]
-    s = make()
-    p = PlainPath(s, export_atom_groups=True, max_neighbor_numbers=3000)
+    p = PlainPath(s, **kw)
     for _ in range(8):  # the dense box starts above the default capacities
         if not p.nl.Check_Overflow({}, 149, s.cell, s.rcell):
             break
         p.update(0, forced=True)
         p.force()
     assert p.nl.stats()["overflow"] == 0
+    return p
 
-    def build_and_force():
-        p.update(0, forced=True)
-        p.force()
 
+def traced_splits():
+    """Every case's split, read from its launched kernels."""
+    import torch
+    out = {}
+    for name, (make, *_) in CASES.items():
+        p = _path(make())
+
+        def build_and_force():
+            p.update(0, forced=True)
+            p.force()
+
+        out[name] = _split(kernel_launches(torch, build_and_force))
+    return out
+
+
+def test_cases_run_the_splits_they_are_for(torch_cuda):
     assert torch_cuda.cuda.get_device_properties(0).multi_processor_count == 148, "the cases' sizes are for 148 SMs"
-    assert _split(kernel_launches(torch_cuda, build_and_force)) == tuple(split)
+    got = in_fresh_process("test_gpu_work_split", "traced_splits")
+    assert {k: tuple(v) for k, v in got.items()} == {k: tuple(split) for k, (_, *split) in CASES.items()}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_split_lists_and_forces(torch_cuda, oracle, name):
+    s = CASES[name][0]()
+    p = _path(s, export_atom_groups=True, max_neighbor_numbers=3000)
     counts, lists = p.nl.host_atom_groups()
     oc, ol = oracle.nl_build(s, mode=1)
     assert np.array_equal(counts, oc)
